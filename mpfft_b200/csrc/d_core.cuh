@@ -1,6 +1,6 @@
 // Device functions of the FP64 conjugate-pair split-radix kernels: the
-// reference's n=8 and n=16 base cases, the 4m2a butterfly and one CTA's
-// shared-memory sub-transform instances.  Shared by the per-launch kernels
+// reference's n=8 and n=16 base cases, the 4m2a butterfly, passes of up to
+// three levels in registers and one CTA's shared-memory sub-transforms.  Shared by the per-launch kernels
 // (d_kernels.cu) and the persistent work-queue kernels (queue_kernels.cu);
 // every file that includes it is compiled with --fmad=false so that no
 // multiply-add is contracted and results stay bit-identical to the reference.
@@ -9,12 +9,9 @@
 #include <cstdint>
 
 #include "mpfft_internal.h"
+#include "sr_chunks.cuh"
 
 namespace mpfft {
-
-struct DConst {
-  double c8, c16a, c16b, c16c, c16d;
-};
 
 // 8-point base case on one part (reference :153-191); v = b1..b8
 __device__ __forceinline__ void d8_part(const DConst &K, const double *x, double *v) {
@@ -88,290 +85,302 @@ __device__ __forceinline__ void d16_part(const DConst &K, const double *x, bool 
   o.c20 = c14 - c16;
 }
 
-// Shared-memory index: the low 4 bits of m XOR-ed with bits 4-7 ^ 8-11 (a
-// permutation inside every 16-aligned block, so a plane needs no padding).
-// Leaves work on 16 (or 8) consecutive elements per thread, levels on
-// consecutive k, the DIT gather on scattered positions; over the whole
-// 4096-point schedule this needs 29 % fewer shared-memory wavefronts than one
-// pad slot per 16 elements (counted by simulating every access of the
-// schedule per half-warp and bank).
-__device__ __forceinline__ int pidx(int m) { return m ^ (((m >> 4) ^ (m >> 8)) & 15); }
-
-// Leaf of size 16 at positions [o, o+16) (reference :213-385), in place.
-__device__ __forceinline__ void d_leaf16(const DConst &K, double *yr, double *yi, int o) {
-  double xr[16], xi[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    xr[j] = yr[pidx(o + j)];
-    xi[j] = yi[pidx(o + j)];
-  }
+// 16-point base case (reference :213-385): x -> out(position, value)
+template <class F>
+__device__ __forceinline__ void d_leaf16(const DConst &K, const double *xr, const double *xi, F out) {
   D16 R, I;
   d16_part(K, xr, false, R);
   d16_part(K, xi, true, I);
   // output stage (reference :350-382)
-  double *r = yr, *i = yi;
-#define P(j) pidx(o + (j))
-  r[P(0)] = R.b5 + R.b11;  r[P(8)] = R.b5 - R.b11;
-  i[P(0)] = I.b5 + I.b11;  i[P(8)] = I.b5 - I.b11;
-  r[P(4)] = R.b6 - I.b12;  r[P(12)] = R.b6 + I.b12;
-  i[P(4)] = I.b6 - R.b12;  i[P(12)] = I.b6 + R.b12;
-  r[P(1)] = R.c9 - I.c17;  r[P(15)] = R.c9 + I.c17;
-  i[P(1)] = I.c9 - R.c17;  i[P(15)] = I.c9 + R.c17;
-  r[P(2)] = R.c1 - I.c3;   r[P(14)] = R.c1 + I.c3;
-  i[P(2)] = I.c1 - R.c3;   i[P(14)] = I.c1 + R.c3;
-  r[P(3)] = R.c12 + I.c20; r[P(13)] = R.c12 - I.c20;
-  i[P(3)] = I.c12 + R.c20; i[P(13)] = I.c12 - R.c20;
-  r[P(5)] = R.c11 - I.c19; r[P(11)] = R.c11 + I.c19;
-  i[P(5)] = I.c11 - R.c19; i[P(11)] = I.c11 + R.c19;
-  r[P(6)] = R.c2 - I.c4;   r[P(10)] = R.c2 + I.c4;
-  i[P(6)] = I.c2 - R.c4;   i[P(10)] = I.c2 + R.c4;
-  r[P(7)] = R.c10 + I.c18; r[P(9)] = R.c10 - I.c18;
-  i[P(7)] = I.c10 + R.c18; i[P(9)] = I.c10 - R.c18;
-#undef P
+  out(0, R.b5 + R.b11, I.b5 + I.b11);
+  out(8, R.b5 - R.b11, I.b5 - I.b11);
+  out(4, R.b6 - I.b12, I.b6 - R.b12);
+  out(12, R.b6 + I.b12, I.b6 + R.b12);
+  out(1, R.c9 - I.c17, I.c9 - R.c17);
+  out(15, R.c9 + I.c17, I.c9 + R.c17);
+  out(2, R.c1 - I.c3, I.c1 - R.c3);
+  out(14, R.c1 + I.c3, I.c1 + R.c3);
+  out(3, R.c12 + I.c20, I.c12 + R.c20);
+  out(13, R.c12 - I.c20, I.c12 - R.c20);
+  out(5, R.c11 - I.c19, I.c11 - R.c19);
+  out(11, R.c11 + I.c19, I.c11 + R.c19);
+  out(6, R.c2 - I.c4, I.c2 - R.c4);
+  out(10, R.c2 + I.c4, I.c2 + R.c4);
+  out(7, R.c10 + I.c18, I.c10 + R.c18);
+  out(9, R.c10 - I.c18, I.c10 - R.c18);
 }
 
-// Leaf of size 8 at positions [o, o+8) (reference :148-212), in place.
-__device__ __forceinline__ void d_leaf8(const DConst &K, double *yr, double *yi, int o) {
-  double xr[8], xi[8], R[8], I[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    xr[j] = yr[pidx(o + j)];
-    xi[j] = yi[pidx(o + j)];
-  }
+// 8-point base case (reference :148-212)
+template <class F>
+__device__ __forceinline__ void d_leaf8(const DConst &K, const double *xr, const double *xi, F out) {
+  double R[8], I[8];
   d8_part(K, xr, R);
   d8_part(K, xi, I);
   // output stage (reference :193-209)
-#define P(j) pidx(o + (j))
-  yr[P(0)] = R[1] + R[0]; yr[P(4)] = R[1] - R[0];
-  yi[P(0)] = I[1] + I[0]; yi[P(4)] = I[1] - I[0];
-  yr[P(1)] = R[4] + I[6]; yr[P(7)] = R[4] - I[6];
-  yi[P(1)] = I[4] - R[6]; yi[P(7)] = I[4] + R[6];
-  yr[P(2)] = R[2] + I[3]; yr[P(6)] = R[2] - I[3];
-  yi[P(2)] = I[2] - R[3]; yi[P(6)] = I[2] + R[3];
-  yr[P(3)] = R[5] - I[7]; yr[P(5)] = R[5] + I[7];
-  yi[P(3)] = I[5] + R[7]; yi[P(5)] = I[5] - R[7];
-#undef P
+  out(0, R[1] + R[0], I[1] + I[0]);
+  out(4, R[1] - R[0], I[1] - I[0]);
+  out(1, R[4] + I[6], I[4] - R[6]);
+  out(7, R[4] - I[6], I[4] + R[6]);
+  out(2, R[2] + I[3], I[2] - R[3]);
+  out(6, R[2] - I[3], I[2] + R[3]);
+  out(3, R[5] - I[7], I[5] + R[7]);
+  out(5, R[5] + I[7], I[5] - R[7]);
 }
 
-// Leaves of size 4, 2, 1 (only when the whole transform has N <= 4).
-__device__ __forceinline__ void d_leaf_small(double *yr, double *yi, int o, int n) {
-  double xr[4], xi[4];
-  for (int j = 0; j < n; ++j) {
-    xr[j] = yr[pidx(o + j)];
-    xi[j] = yi[pidx(o + j)];
-  }
-  if (n == 4) {  // reference :121-147
-    const double er = xr[0] + xr[2], fr = xr[0] - xr[2], gr = xr[1] + xr[3], hr = xr[1] - xr[3];
-    const double ei = xi[0] + xi[2], fi = xi[0] - xi[2], gi = xi[1] + xi[3], hi = xi[1] - xi[3];
-    yr[pidx(o + 0)] = er + gr; yr[pidx(o + 1)] = fr + hi; yr[pidx(o + 2)] = er - gr; yr[pidx(o + 3)] = fr - hi;
-    yi[pidx(o + 0)] = ei + gi; yi[pidx(o + 1)] = fi - hr; yi[pidx(o + 2)] = ei - gi; yi[pidx(o + 3)] = fi + hr;
-  } else if (n == 2) {  // reference :108-120
-    yr[pidx(o)] = xr[0] + xr[1]; yr[pidx(o + 1)] = xr[0] - xr[1];
-    yi[pidx(o)] = xi[0] + xi[1]; yi[pidx(o + 1)] = xi[0] - xi[1];
-  }
-}
-
-// 4m2a butterfly k of a node of size n at y[off..) (reference :392-427)
-// (outputs to the planes exchanged when swap_out: the last launch of an inverse)
-__device__ __forceinline__ void d_butterfly(double *yr, double *yi, size_t stride, int off, int k, int q,
-                                            double w_r, double w_i, double scale, bool swap_out = false) {
-  double *r0 = yr + (size_t)(off + k) * stride, *i0 = yi + (size_t)(off + k) * stride;
-  const size_t qs = (size_t)q * stride;
-  const double u0r = r0[0], u1r = r0[qs], zpr = r0[2 * qs], zmr = r0[3 * qs];
-  const double u0i = i0[0], u1i = i0[qs], zpi = i0[2 * qs], zmi = i0[3 * qs];
-  const double pr = w_r * zpr + w_i * zpi, pi = w_r * zpi - w_i * zpr;
-  const double mr = w_r * zmr - w_i * zmi, mi = w_r * zmi + w_i * zmr;
+// 4m2a butterfly (reference :392-427) on values in registers: (U0, U1, Z+, Z-)
+// -> the outputs that go to the same four positions.  A complex value is a
+// double2 (x real, y imaginary), a twiddle w = (cos, sin).
+__device__ __forceinline__ void d_bfly(double2 &u0, double2 &u1, double2 &zp, double2 &zm, double2 w) {
+  const double pr = w.x * zp.x + w.y * zp.y, pi = w.x * zp.y - w.y * zp.x;
+  const double mr = w.x * zm.x - w.y * zm.y, mi = w.x * zm.y + w.y * zm.x;
   const double sr = pr + mr, si = pi + mi, dr = pr - mr, di = pi - mi;
-  if (swap_out) {
-    double *t = r0;
-    r0 = i0;
-    i0 = t;
-  }
-  r0[0] = (u0r + sr) * scale;
-  r0[2 * qs] = (u0r - sr) * scale;
-  r0[qs] = (u1r + di) * scale;
-  r0[3 * qs] = (u1r - di) * scale;
-  i0[0] = (u0i + si) * scale;
-  i0[2 * qs] = (u0i - si) * scale;
-  i0[qs] = (u1i - dr) * scale;
-  i0[3 * qs] = (u1i + dr) * scale;
+  const double2 a = u0, b = u1;
+  u0 = make_double2(a.x + sr, a.y + si);
+  zp = make_double2(a.x - sr, a.y - si);
+  u1 = make_double2(b.x + di, b.y - dr);
+  zm = make_double2(b.x - di, b.y + dr);
 }
 
-// 4m2a butterfly on values in registers: (U0, U1, Z+, Z-) -> the outputs that
-// go to the same four positions (the operations of d_butterfly)
-struct DCplx {
-  double r, i;
+// R levels (node sizes 4u, 8u, 16u) of one column: v[j] = y[base + k + j*u],
+// j < 2^(R+1), of the chunk of 2^(R+1)*u positions at `base`.  The chunk is
+// one node of its own size (big), or a pair of nodes of half of it
+// (sr_chunk_big); nodes of size 2u and below are complete.  Butterfly k + i*u of
+// a node of size n only touches positions k mod u, so the column is closed
+// under all its levels and they run in registers: the points cross memory once
+// per R levels.  tw: per-level twiddles (sr_level_tw), all k.
+template <int R>
+__device__ __forceinline__ void d_levels(double2 (&v)[2 << R], bool big, const double2 *__restrict__ tw, int u, int k) {
+  const double2 *t4 = tw + sr_level_tw(4 * u), *t8 = tw + sr_level_tw(8 * u), *t16 = tw + sr_level_tw(16 * u);
+  if constexpr (R == 1) {
+    if (big) d_bfly(v[0], v[1], v[2], v[3], __ldg(t4 + k));
+  } else if constexpr (R == 2) {
+    const double2 w4 = __ldg(t4 + k);
+    d_bfly(v[0], v[1], v[2], v[3], w4);
+    if (big) {
+      d_bfly(v[0], v[2], v[4], v[6], __ldg(t8 + k));
+      d_bfly(v[1], v[3], v[5], v[7], __ldg(t8 + k + u));
+    } else {
+      d_bfly(v[4], v[5], v[6], v[7], w4);
+    }
+  } else {
+    const double2 w4 = __ldg(t4 + k), w8a = __ldg(t8 + k), w8b = __ldg(t8 + k + u);
+    d_bfly(v[0], v[1], v[2], v[3], w4);
+    d_bfly(v[8], v[9], v[10], v[11], w4);
+    d_bfly(v[0], v[2], v[4], v[6], w8a);
+    d_bfly(v[1], v[3], v[5], v[7], w8b);
+    if (big) {
+      d_bfly(v[12], v[13], v[14], v[15], w4);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) d_bfly(v[i], v[i + 4], v[i + 8], v[i + 12], __ldg(t16 + k + i * u));
+    } else {
+      d_bfly(v[8], v[10], v[12], v[14], w8a);
+      d_bfly(v[9], v[11], v[13], v[15], w8b);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// one CTA's sub-transforms: G chunks of T = 2^lgT points in shared memory
+// ---------------------------------------------------------------------------
+//
+// SINGLE: T = N and the chunks are whole signals b0 .. b0+G-1.  Otherwise the
+// chunks are those of G consecutive input classes c0 .. of signal b0 (chunk m
+// = output positions [mT, (m+1)T), whose inputs are x[c + j*(N/T)] for its
+// class c, so neighbouring classes share 32-byte sectors).
+//
+// Base cases straight from global memory: one thread per 16 output positions
+// (a leaf of 16 points or a pair of leaves of 8, either way 16 inputs x[c' + j*(N/16)]
+// of one class c'), then passes of up to three levels (d_levels), the last of
+// which writes its outputs to global memory.  Shared memory is crossed once
+// per pass: 3.5 times (in + out) at T = 4096 against about ten for two levels
+// per pass after a separate gather.  Measured, 2^24 points in and out (us, that
+// form / this one): N = 64 272 / 116, 1024 268 / 113, 4096 305 / 125 (4.3 TB/s
+// of the 6.5 TB/s copy rate; two CTAs of 256 threads per SM, 16 points a thread,
+// 122 registers), 65536 724 / 303, 2^20 963 / 439.
+//
+// Shared positions m are swizzled (low 3 bits ^= bits 3-5 ^ 6-8 ^ 9-11, 16-byte
+// elements): columns are 8 or more consecutive k, conflict-free; the base
+// cases' stores are scattered, and the host orders the slots so that they
+// average 1.0-1.4 wavefronts per ideal one (counted by simulating them).
+struct DSubArgs {
+  const double *in;
+  double *out;
+  int B, b0, c0, G;
+  double scale;       // applied to the outputs when `final`
+  bool final;         // these outputs are the transform's
+  bool swap_in, swap_out;
 };
-__device__ __forceinline__ void d_bfly_vals(DCplx &u0, DCplx &u1, DCplx &zp, DCplx &zm, double w_r, double w_i,
-                                            double scale) {
-  const double pr = w_r * zp.r + w_i * zp.i, pi = w_r * zp.i - w_i * zp.r;
-  const double mr = w_r * zm.r - w_i * zm.i, mi = w_r * zm.i + w_i * zm.r;
-  const double sr = pr + mr, si = pi + mi, dr = pr - mr, di = pi - mi;
-  const DCplx a = u0, b = u1;
-  u0 = DCplx{(a.r + sr) * scale, (a.i + si) * scale};
-  zp = DCplx{(a.r - sr) * scale, (a.i - si) * scale};
-  u1 = DCplx{(b.r + di) * scale, (b.i - dr) * scale};
-  zm = DCplx{(b.r - di) * scale, (b.i + dr) * scale};
-}
 
-// 4m2a butterfly in shared memory (padded indices)
-__device__ __forceinline__ void d_butterfly_smem(double *yr, double *yi, int off, int k, int q, double w_r,
-                                                 double w_i, double scale) {
-  const int a[4] = {pidx(off + k), pidx(off + k + q), pidx(off + k + 2 * q), pidx(off + k + 3 * q)};
-  DCplx v[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = DCplx{yr[a[j]], yi[a[j]]};
-  d_bfly_vals(v[0], v[1], v[2], v[3], w_r, w_i, scale);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) yr[a[j]] = v[j].r, yi[a[j]] = v[j].i;
-}
+__device__ __forceinline__ int d_swz(int m) { return m ^ (((m >> 3) ^ (m >> 6) ^ (m >> 9)) & 7); }
 
-// Two levels of one node in shared memory: butterfly k of the first child X
-// (size n, q = n/4, at the node's offset) and butterflies k and k+q of the node
-// Y (size 2n), whose U inputs are exactly X's four outputs -- they stay in
-// registers between the two levels.  wx: X's twiddle; wy0, wy1: Y's for k and
-// k+q; scale applies to Y's outputs.
-__device__ __forceinline__ void d_bfly_pair_smem(double *yr, double *yi, int off, int k, int q, double wx_r,
-                                                 double wx_i, double wy0_r, double wy0_i, double wy1_r,
-                                                 double wy1_i, double scale) {
-  int a[8];
-  DCplx v[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    a[j] = pidx(off + k + j * q);
-    v[j] = DCplx{yr[a[j]], yi[a[j]]};
-  }
-  d_bfly_vals(v[0], v[1], v[2], v[3], wx_r, wx_i, 1.0);
-  d_bfly_vals(v[0], v[2], v[4], v[6], wy0_r, wy0_i, scale);
-  d_bfly_vals(v[1], v[3], v[5], v[7], wy1_r, wy1_i, scale);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) yr[a[j]] = v[j].r, yi[a[j]] = v[j].i;
-}
-
-// One CTA = G instances (sub-transform root x signal) entirely in shared
-// memory.  SINGLE: N < 4096, one root per signal, G signals per CTA, all with
-// the big schedule.  Otherwise G = 1 and the CTA's root may be of size T or
-// T/2.  Per instance: gather the root's input sequence in input order
-// (coalesced reads) into DIT positions, leaves, levels, then write the outputs
-// once.  The twiddles the levels need, LUT[m*(N/T)] for m < T/4, are read
-// through L1 (a few KB, shared by all CTAs).
-// The instances of one CTA: G_here signals b0.. of root rt (SINGLE: the whole
-// transform, several signals per CTA; otherwise one signal, and the root may
-// be of size T or T/2), sm the CTA's shared memory.
 template <bool SINGLE>
-__device__ __forceinline__ void d_sub_instances(const double *__restrict__ in, double *__restrict__ out, int N, int B,
-                                                int b0, int G_here, SubRoot rt, const SubSchedule &big,
-                                                const SubSchedule &small, const double *__restrict__ wr,
-                                                const double *__restrict__ wi, const DConst &K, double scale,
-                                                int swap_in, int swap_out, double *sm) {
-  const int Tmax = big.size;
-  const int lgT = 31 - __clz(Tmax);
-  const int istride = 2 * Tmax;  // doubles per instance: real plane, imaginary plane
-  const int tws = N / Tmax;                  // twiddle table stride of this sub-transform
-  const bool is_big = SINGLE || rt.size == Tmax;
-  const int T = rt.size;
-  const int *perm = is_big ? big.perm : small.perm;
-  const Leaf *leaves = is_big ? big.leaves : small.leaves;
-  const int nleaves = is_big ? big.nleaves : small.nleaves;
-  const int n16 = is_big ? big.nleaf16 : small.nleaf16, n8 = is_big ? big.nleaf8 : small.nleaf8;
-  const int nlevels = is_big ? big.nlevels : small.nlevels;
-  // gather: element j of instance g to DIT position perm[j]; 8 elements per
-  // thread are loaded before any is stored, so their latencies overlap
-  const int total = G_here << lgT;
-  for (int e0 = 0; e0 < total; e0 += 8 * (int)blockDim.x) {
-    double vr[8], vi[8];
-    int dst[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int e = e0 + u * (int)blockDim.x + (int)threadIdx.x;
-      const int g = e >> lgT, j = e & (Tmax - 1);
-      dst[u] = -1;
-      if (e < total && (SINGLE || j < T)) {
-        int idx = rt.sn + j * rt.s;
-        if (idx < 0) idx += N;
-        const size_t b = (size_t)(b0 + g);
-        vr[u] = in[(swap_in ? (size_t)B + b : b) * N + idx];
-        vi[u] = in[(swap_in ? b : (size_t)B + b) * N + idx];
-        dst[u] = g * istride + pidx(perm[j]);
+__device__ __forceinline__ int d_chunk_of(const DSubTab &S, const DSubArgs &A, int g) {
+  return SINGLE ? 0 : __ldg(&S.chunks[A.c0 + g].chunk);
+}
+
+template <int LGT, bool SINGLE>
+__device__ __forceinline__ void d_sub_leaves(const DSubTab &S, const DSubArgs &A, double2 *sm) {
+  constexpr int T = 1 << LGT, kSlots = T / 16;
+  const int step = S.N >> 4;  // input stride of a 16-point leaf
+  for (int e = threadIdx.x; e < A.G * kSlots; e += blockDim.x) {
+    const int g = SINGLE ? e / kSlots : e % A.G;
+    int s = SINGLE ? e % kSlots : e / A.G;
+    int half = 0, sna = 0, rs = 1, chunk = 0;
+    const SrLeafSlot *tab = S.slots[0];
+    if (!SINGLE) {
+      const SrChunk ch = S.chunks[A.c0 + g];
+      chunk = ch.chunk;
+      sna = ch.sna;
+      rs = S.N >> LGT;
+      if (!sr_chunk_big(chunk)) {  // a pair of sub-transforms of T/2 points
+        tab = S.slots[1];
+        rs *= 2;
+        half = s >= kSlots / 2;
+        s -= half ? kSlots / 2 : 0;
+        if (half) sna = ch.snb;
       }
     }
+    const SrLeafSlot L = tab[s];
+    const int m = half * (kSlots / 2) + L.m;  // 16-point block of the chunk
+    const bool big = sr_chunk_big(chunk * kSlots + m);
+    // leaf input j: sn + j*stride, j = 0 wrapped when negative
+    const int a0 = sna + L.sna * rs, b0 = sna + L.snb * rs;
+    const size_t b = (size_t)(SINGLE ? A.b0 + g : A.b0);
+    const double *pr = A.in + (A.swap_in ? (size_t)A.B + b : b) * S.N;
+    const double *pi = A.in + (A.swap_in ? b : (size_t)A.B + b) * S.N;
+    double xr[16], xi[16];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (dst[u] >= 0) {
-        sm[dst[u]] = vr[u];
-        sm[dst[u] + Tmax] = vi[u];
+    for (int j = 0; j < 16; ++j) {
+      int idx = big ? a0 + j * step : (j < 8 ? a0 + 2 * j * step : b0 + 2 * (j - 8) * step);
+      if ((j == 0 || j == 8) && idx < 0) idx += S.N;
+      xr[j] = pr[idx];
+      xi[j] = pi[idx];
+    }
+    const int at = d_swz(g * T + 16 * m);  // position p of the block is at ^ d_swz(p)
+    if (big) {
+      d_leaf16(S.K, xr, xi, [&](int p, double r, double i) { sm[at ^ d_swz(p)] = make_double2(r, i); });
+    } else {
+      d_leaf8(S.K, xr, xi, [&](int p, double r, double i) { sm[at ^ d_swz(p)] = make_double2(r, i); });
+      d_leaf8(S.K, xr + 8, xi + 8, [&](int p, double r, double i) { sm[at ^ d_swz(p + 8)] = make_double2(r, i); });
+    }
+  }
+}
+
+// R levels of every chunk of 2^(R+1)*u positions, u = 2^LGU; LAST: the outputs go to global memory
+template <int LGT, int LGU, int R, bool LAST, bool SINGLE>
+__device__ __forceinline__ void d_sub_pass(const DSubTab &S, const DSubArgs &A, double2 *sm) {
+  constexpr int u = 1 << LGU, M = 2 << R, lgc = LGU + R + 1, nch = 1 << (LGT - lgc);
+  __syncthreads();
+  for (int e = threadIdx.x; e < A.G << (LGT - R - 1); e += blockDim.x) {
+    const int k = e & (u - 1), c = e >> LGU, g = c / nch;
+    const int chunk = d_chunk_of<SINGLE>(S, A, g);
+    const int at = d_swz((c << lgc) + k);  // the swizzle is linear over xor: position j*u is at ^ d_swz(j*u)
+    double2 v[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) v[j] = sm[at ^ d_swz(j << LGU)];
+    d_levels<R>(v, sr_chunk_big(chunk * nch + c % nch), S.tw, u, k);
+    if (!LAST) {
+#pragma unroll
+      for (int j = 0; j < M; ++j) sm[at ^ d_swz(j << LGU)] = v[j];
+    } else {
+      const size_t b = (size_t)(SINGLE ? A.b0 + g : A.b0);
+      const size_t p = ((size_t)chunk << LGT) + ((c % nch) << lgc) + k;
+      double *qr = A.out + (A.swap_out ? (size_t)A.B + b : b) * S.N + p;
+      double *qi = A.out + (A.swap_out ? b : (size_t)A.B + b) * S.N + p;
+      const double sc = A.final ? A.scale : 1.0;
+#pragma unroll
+      for (int j = 0; j < M; ++j) {
+        qr[j << LGU] = v[j].x * sc;
+        qi[j << LGU] = v[j].y * sc;
       }
+    }
+  }
+}
+
+template <int LGT, bool SINGLE>
+__device__ __forceinline__ void d_sub_transform(const DSubTab &S, const DSubArgs &A, double2 *sm) {
+  static_assert(LGT >= 5 && LGT <= 12, "sub-transforms of 32 to 4096 points");
+  d_sub_leaves<LGT, SINGLE>(S, A, sm);
+  constexpr int R1 = LGT - 4 < 3 ? LGT - 4 : 3;
+  d_sub_pass<LGT, 3, R1, (LGT <= 7), SINGLE>(S, A, sm);
+  if constexpr (LGT > 7) {
+    constexpr int R2 = LGT - 7 < 3 ? LGT - 7 : 3;
+    d_sub_pass<LGT, 6, R2, (LGT <= 10), SINGLE>(S, A, sm);
+  }
+  if constexpr (LGT > 10) d_sub_pass<LGT, 9, LGT - 10, true, SINGLE>(S, A, sm);
+}
+
+// Transforms of N <= 16 points (one base case): G signals b0 .. through
+// shared memory, so that the global accesses are contiguous.
+__device__ __forceinline__ void d_tiny(const DSubTab &S, const DSubArgs &A, double2 *sm) {
+  const int N = S.N, total = A.G * N;
+  const size_t at = (size_t)A.b0 * N, im = (size_t)A.B * N;
+  for (int e = threadIdx.x; e < total; e += blockDim.x)
+    sm[d_swz(e)] = make_double2(A.in[at + e + (A.swap_in ? im : 0)], A.in[at + e + (A.swap_in ? 0 : im)]);
+  __syncthreads();
+  for (int g = threadIdx.x; g < A.G; g += blockDim.x) {
+    const int o = g * N;
+    double xr[16], xi[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < N) {
+        const double2 v = sm[d_swz(o + j)];
+        xr[j] = v.x;
+        xi[j] = v.y;
+      }
+    auto put = [&](int p, double r, double i) { sm[d_swz(o + p)] = make_double2(r * A.scale, i * A.scale); };
+    if (N == 16) {
+      d_leaf16(S.K, xr, xi, put);
+    } else if (N == 8) {
+      d_leaf8(S.K, xr, xi, put);
+    } else if (N == 4) {  // reference :121-147
+      const double er = xr[0] + xr[2], fr = xr[0] - xr[2], gr = xr[1] + xr[3], hr = xr[1] - xr[3];
+      const double ei = xi[0] + xi[2], fi = xi[0] - xi[2], gi = xi[1] + xi[3], hi = xi[1] - xi[3];
+      put(0, er + gr, ei + gi);
+      put(1, fr + hi, fi - hr);
+      put(2, er - gr, ei - gi);
+      put(3, fr - hi, fi + hr);
+    } else if (N == 2) {  // reference :108-120
+      put(0, xr[0] + xr[1], xi[0] + xi[1]);
+      put(1, xr[0] - xr[1], xi[0] - xi[1]);
+    } else {
+      put(0, xr[0], xi[0]);
+    }
   }
   __syncthreads();
-  // leaves, grouped by size: 16-point, then 8-point, then (N <= 4 only) smaller
-  for (int e = threadIdx.x; e < G_here * nleaves; e += blockDim.x) {
-    const int g = SINGLE ? e / nleaves : 0, l = SINGLE ? e - g * nleaves : e;
-    double *yr = sm + (size_t)g * istride, *yi = yr + Tmax;
-    const Leaf lf = leaves[l];
-    if (l < n16) d_leaf16(K, yr, yi, lf.out);
-    else if (l < n16 + n8) d_leaf8(K, yr, yi, lf.out);
-    else d_leaf_small(yr, yi, lf.out, lf.n);
+  for (int e = threadIdx.x; e < total; e += blockDim.x) {
+    const double2 v = sm[d_swz(e)];
+    A.out[at + e + (A.swap_out ? im : 0)] = v.x;
+    A.out[at + e + (A.swap_out ? 0 : im)] = v.y;
   }
-  if (nlevels == 0 && scale != 1.0) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < (G_here << lgT); e += blockDim.x) {
-      const int g = e >> lgT, m = e & (Tmax - 1);
-      double *yr = sm + (size_t)g * istride, *yi = yr + Tmax;
-      yr[pidx(m)] *= scale;
-      yi[pidx(m)] *= scale;
-    }
+}
+
+// ---------------------------------------------------------------------------
+// R levels above the sub-transforms, in place in global memory: column k of
+// chunk c (of 2^(R+1)*u positions) of signal b
+// ---------------------------------------------------------------------------
+template <int R>
+__device__ __forceinline__ void d_upper_column(double *__restrict__ y, int N, int B, int lgu, int b, int c, int k,
+                                               const double2 *__restrict__ tw, double scale, bool swap_out) {
+  constexpr int M = 2 << R;
+  const size_t u = (size_t)1 << lgu, p = ((size_t)c << (lgu + R + 1)) + k;
+  double *yr = y + (size_t)b * N + p, *yi = y + ((size_t)B + b) * N + p;
+  double2 v[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) v[j] = make_double2(yr[j * u], yi[j * u]);
+  d_levels<R>(v, sr_chunk_big(c), tw, (int)u, k);
+  double *qr = swap_out ? yi : yr, *qi = swap_out ? yr : yi;
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    qr[j * u] = v[j].x * scale;
+    qi[j * u] = v[j].y * scale;
   }
-  // levels (the small schedule's levels are the big one's minus the last),
-  // two per pass: each node of the upper level with its first child, then the
-  // lower level's other nodes; an odd top level runs alone
-  const SubSchedule &S = is_big ? big : small;
-  for (int lv = 0; lv < nlevels; ++lv) {
-    __syncthreads();
-    const int n = big.level_n[lv], q = n >> 2, lgq = 29 - __clz(n);
-    if (lv + 1 < nlevels) {
-      const int cy = S.level_count[lv + 1], cu = S.pair_count[lv];
-      const int *ynodes = S.node_off + S.level_start[lv + 1], *unodes = S.pair_nodes + S.pair_start[lv];
-      const int per = (cy + cu) * q;
-      const double sc = lv + 1 == nlevels - 1 ? scale : 1.0;
-      for (int e = threadIdx.x; e < G_here * per; e += blockDim.x) {
-        const int g = SINGLE ? e / per : 0, t = SINGLE ? e - g * per : e;
-        const int node = t >> lgq, k = t & (q - 1);
-        const int km = k << (lgT - (lgq + 2));  // k * (T/n)
-        double *yr = sm + (size_t)g * istride, *yi = yr + Tmax;
-        if (node < cy) {
-          const int ky0 = k << (lgT - (lgq + 3)), ky1 = (k + q) << (lgT - (lgq + 3));  // k * (T/2n), (k+q) * (T/2n)
-          d_bfly_pair_smem(yr, yi, ynodes[node], k, q, __ldg(wr + (size_t)km * tws), __ldg(wi + (size_t)km * tws),
-                           __ldg(wr + (size_t)ky0 * tws), __ldg(wi + (size_t)ky0 * tws),
-                           __ldg(wr + (size_t)ky1 * tws), __ldg(wi + (size_t)ky1 * tws), sc);
-        } else {
-          d_butterfly_smem(yr, yi, unodes[node - cy], k, q, __ldg(wr + (size_t)km * tws),
-                           __ldg(wi + (size_t)km * tws), 1.0);
-        }
-      }
-      ++lv;
-      continue;
-    }
-    const int cnt = is_big ? big.level_count[lv] : small.level_count[lv];
-    const int *nodes = (is_big ? big.node_off : small.node_off) + (is_big ? big.level_start[lv] : small.level_start[lv]);
-    const int per = cnt * q;
-    const double sc = lv == nlevels - 1 ? scale : 1.0;
-    for (int e = threadIdx.x; e < G_here * per; e += blockDim.x) {
-      const int g = SINGLE ? e / per : 0, t = SINGLE ? e - g * per : e;
-      const int node = t >> lgq, k = t & (q - 1);
-      const int km = k << (lgT - (lgq + 2));  // k * (T/n)
-      double *yr = sm + (size_t)g * istride, *yi = yr + Tmax;
-      d_butterfly_smem(yr, yi, nodes[node], k, q, __ldg(wr + (size_t)km * tws), __ldg(wi + (size_t)km * tws), sc);
-    }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < (G_here << lgT); e += blockDim.x) {
-    const int g = e >> lgT, m = e & (Tmax - 1);
-    if (!SINGLE && m >= T) continue;
-    const int b = b0 + g;
-    const double *yr = sm + (size_t)g * istride, *yi = yr + Tmax;
-    out[(swap_out ? (size_t)B + b : (size_t)b) * N + rt.out + m] = yr[pidx(m)];
-    out[(swap_out ? (size_t)b : (size_t)B + b) * N + rt.out + m] = yi[pidx(m)];
-  }
+}
+
+// levels above the sub-transforms per pass: nl levels in the fewest passes of at most three, evenly
+__host__ __device__ inline int d_upper_levels(int nl) {
+  const int passes = (nl + 2) / 3;
+  return passes ? (nl + passes - 1) / passes : 0;
 }
 
 }  // namespace mpfft

@@ -7,14 +7,13 @@
 // association.  This file is compiled with --fmad=false so no multiply-add is
 // contracted into an FMA (the reference's x86-64 build has no FMA either).
 //
-// Schedule: the reference's recursion tree, cut at T = min(N, 4096) points.
-// Every maximal node of size <= T (size T or T/2) is one shared-memory
-// sub-transform: one CTA gathers its input sequence in DIT order (so every
-// leaf's inputs already sit where its outputs go), runs the leaves (n = 16 and
-// 8; the whole transform for N <= 16) and all levels up to the node in place
-// in shared memory, and writes the node's outputs once.  Levels above T run
-// one launch per node size in global memory.  For N <= 4096 a transform is one
-// launch that reads its input once and writes its output once.
+// Schedule: the reference's recursion tree, cut at T <= 4096 points.  Chunks
+// of T output positions run in shared memory (d_core.cuh): base cases of 16
+// and 8 points straight from global memory, then passes of up to three levels
+// whose points stay in registers, the last one written out.  Levels above T
+// run three (or two) per launch in global memory, again in registers.  For
+// N <= 4096 a transform is one launch that reads its input once and writes its
+// output once.
 //
 // Layout: word (c, b, p) at base[(c*B + b)*N + p] -- each signal contiguous.
 #include <algorithm>
@@ -25,39 +24,56 @@
 
 namespace mpfft {
 
-template <bool SINGLE>
-__global__ void __launch_bounds__(256, 3) d_sub_kernel(const double *__restrict__ in, double *__restrict__ out, int N,
-                                                        int B, const SubRoot *__restrict__ roots, int nroots, int G,
-                                                        SubSchedule big, SubSchedule small,
-                                                        const double *__restrict__ wr, const double *__restrict__ wi,
-                                                        DConst K, double scale, int swap_in, int swap_out) {
-  extern __shared__ double sm[];
+template <int LGT, bool SINGLE>
+__global__ void __launch_bounds__(256, 2) d_sub_kernel(const __grid_constant__ DSubTab S, DSubArgs A, int groups) {
+  extern __shared__ __align__(16) double2 d_smem[];
+  const int g = A.G;
   if (SINGLE) {
-    const int b0 = blockIdx.x * G;
-    d_sub_instances<true>(in, out, N, B, b0, min(G, B - b0), roots[0], big, small, wr, wi, K, scale, swap_in, swap_out,
-                          sm);
+    A.b0 = blockIdx.x * g;
+    A.G = min(g, A.B - A.b0);
   } else {
-    d_sub_instances<false>(in, out, N, B, blockIdx.x / nroots, 1, roots[blockIdx.x % nroots], big, small, wr, wi, K,
-                           scale, swap_in, swap_out, sm);
+    A.b0 = blockIdx.x / groups;
+    A.c0 = (blockIdx.x % groups) * g;
+    A.G = min(g, S.nchunks - A.c0);
   }
+  d_sub_transform<LGT, SINGLE>(S, A, d_smem);
 }
 
-// 4m2a butterflies of all nodes of size n above the shared-memory
-// sub-transforms; consecutive threads are consecutive k of one signal.
-__global__ void __launch_bounds__(256) d_level_kernel(double *__restrict__ y, int N, int B, int n,
-                                                       const int *__restrict__ node_off, int nnodes,
-                                                       const double *__restrict__ wr, const double *__restrict__ wi,
-                                                       double scale, int swap_out) {
-  const int q = n >> 2;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nnodes * q * B) return;
-  const int k = (int)(t % q);
-  const long long r = t / q;
-  const int node = (int)(r % nnodes);
-  const int b = (int)(r / nnodes);
-  const int kn = k * (N / n);
-  d_butterfly(y + (size_t)b * N, y + ((size_t)B + b) * N, 1, node_off[node], k, q, wr[kn], wi[kn], scale,
-              swap_out != 0);
+__global__ void __launch_bounds__(256) d_tiny_kernel(const __grid_constant__ DSubTab S, DSubArgs A) {
+  extern __shared__ __align__(16) double2 d_smem[];
+  A.b0 = blockIdx.x * A.G;
+  A.G = min(A.G, A.B - A.b0);
+  d_tiny(S, A, d_smem);
+}
+
+// R levels above the sub-transforms: one thread per column (d_upper_column),
+// consecutive threads consecutive k of one chunk of one signal.  Memory-bound:
+// three levels cross memory once instead of three times (one 2^20-point signal
+// 100 -> 39 us, five launches instead of nine).
+template <int R>
+__global__ void __launch_bounds__(256, 2) d_upper_kernel(double *__restrict__ y, int N, int B, int lgu, int lgnch,
+                                                         const double2 *__restrict__ tw, double scale, int swap_out) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long r = e >> lgu;
+  const long long b = r >> lgnch;
+  if (b >= B) return;
+  d_upper_column<R>(y, N, B, lgu, (int)b, (int)(r & ((1 << lgnch) - 1)), (int)(e & ((1 << lgu) - 1)), tw, scale,
+                    swap_out != 0);
+}
+
+__global__ void __launch_bounds__(256) d_level_tw_kernel(const double *__restrict__ wr, const double *__restrict__ wi,
+                                                         int N, double2 *__restrict__ tw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of the table
+  if (i >= N / 2 - 8) return;
+  const int q = 1 << (31 - __clz(i + 8));  // n/4 of its level: entries q-8 .. 2q-9
+  const int k = i + 8 - q;
+  const size_t kn = (size_t)k * (N / (4 * q));
+  tw[i] = make_double2(wr[kn], wi[kn]);
+}
+
+cudaError_t d_build_level_tw(const double *wr, const double *wi, int N, double2 *tw, cudaStream_t s) {
+  d_level_tw_kernel<<<(N / 2 + 255) / 256, 256, 0, s>>>(wr, wi, N, tw);
+  return cudaGetLastError();
 }
 
 // Split step of the FP64 real transforms (n = 2M real points; layouts [c][b][k]).
@@ -134,44 +150,72 @@ cudaError_t d_real_split(bool forward, const double *in, double *out, int M, int
   return cudaGetLastError();
 }
 
-// instances of the shared-memory kernel per CTA and its dynamic shared memory
-static int d_sub_instances(const DDeviceTables &T) {
-  if (T.nroots != 1) return 1;
-  const int per = 2 * T.sub[0].size;
-  return std::max(1, std::min(kDSubMax / std::max(T.sub[0].size, 1), 8192 / per));
+template <int LGT, bool SINGLE>
+static cudaError_t d_sub_launch(const DSubTab &S, DSubArgs A, cudaStream_t s) {
+  constexpr int T = 1 << LGT;
+  // Chunks per CTA: as many as fit, but no more than leave two CTAs for every
+  // SM (a small batch spread over more CTAs finishes earlier).
+  const long long inst = SINGLE ? A.B : (long long)S.nchunks * A.B;
+  int g = kDSubMax / T;
+  while (g > 1 && inst / g < 2 * 148) g /= 2;
+  A.G = g;
+  const size_t smem = (size_t)g * T * sizeof(double2);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(d_sub_kernel<LGT, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kDSubMax * (int)sizeof(double2));
+    if (e != cudaSuccess) return e;
+  }
+  const int threads = std::min(256, std::max(32, g * T / 16));
+  const int groups = SINGLE ? 1 : (S.nchunks + g - 1) / g;
+  const long long ctas = SINGLE ? ((long long)A.B + g - 1) / g : (long long)groups * A.B;
+  d_sub_kernel<LGT, SINGLE><<<(unsigned)ctas, threads, smem, s>>>(S, A, groups);
+  return cudaGetLastError();
 }
 
 cudaError_t d_run_transform(const DDeviceTables &T, const double *in, double *out, int B, double scale,
                             cudaStream_t s, bool swap_in, bool swap_out) {
-  const DConst K{T.c8, T.c16a, T.c16b, T.c16c, T.c16d};
-  const int size = T.sub[0].size;
-  const int G = d_sub_instances(T);
-  const size_t smem = ((size_t)G * 2 * size) * sizeof(double);
-  static bool attr_set = false;  // idempotent; benign race
-  if (!attr_set) {
-    cudaFuncSetAttribute(d_sub_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    cudaFuncSetAttribute(d_sub_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    attr_set = true;
+  const DSubTab &S = T.d;
+  const int nl = S.N > 16 ? 31 - __builtin_clz((unsigned)S.nchunks) : 0;  // levels above the sub-transforms
+  DSubArgs A{in, out, B, 0, 0, 0, scale, nl == 0, swap_in, swap_out && nl == 0};
+  cudaError_t e = cudaSuccess;
+  if (S.N <= 16) {
+    A.G = 2048 / S.N;
+    d_tiny_kernel<<<(unsigned)((B + A.G - 1) / A.G), 256, 2048 * sizeof(double2), s>>>(S, A);
+    return cudaGetLastError();
   }
-  const bool final_sub = T.upper.nlevels == 0;
-  if (T.nroots == 1) {
-    const int blocks = (B + G - 1) / G;
-    d_sub_kernel<true><<<blocks, 256, smem, s>>>(in, out, T.N, B, T.roots, T.nroots, G, T.sub[0], T.sub[1], T.wr,
-                                                 T.wi, K, final_sub ? scale : 1.0, swap_in, final_sub && swap_out);
+#define MPFFT_D_CASE(LL, SINGLE)           \
+  case LL:                                 \
+    e = d_sub_launch<LL, SINGLE>(S, A, s); \
+    break;
+  if (S.nchunks == 1) {
+    switch (S.lgT) {
+      MPFFT_D_CASE(5, true) MPFFT_D_CASE(6, true) MPFFT_D_CASE(7, true) MPFFT_D_CASE(8, true)
+      MPFFT_D_CASE(9, true) MPFFT_D_CASE(10, true) MPFFT_D_CASE(11, true) MPFFT_D_CASE(12, true)
+      default: return cudaErrorInvalidValue;
+    }
   } else {
-    d_sub_kernel<false><<<T.nroots * B, 256, smem, s>>>(in, out, T.N, B, T.roots, T.nroots, 1, T.sub[0], T.sub[1],
-                                                        T.wr, T.wi, K, final_sub ? scale : 1.0, swap_in,
-                                                        final_sub && swap_out);
+    switch (S.lgT) {
+      MPFFT_D_CASE(10, false) MPFFT_D_CASE(11, false) MPFFT_D_CASE(12, false)
+      default: return cudaErrorInvalidValue;
+    }
   }
-  for (int lv = 0; lv < T.upper.nlevels; ++lv) {
-    const int threads = 256;
-    const int n = T.upper.level_n[lv];
-    const long long total = (long long)T.upper.level_count[lv] * (n / 4) * B;
-    const int lblocks = (int)((total + threads - 1) / threads);
-    d_level_kernel<<<lblocks, threads, 0, s>>>(out, T.N, B, n, T.upper.node_off + T.upper.level_start[lv],
-                                               T.upper.level_count[lv], T.wr, T.wi,
-                                               lv == T.upper.nlevels - 1 ? scale : 1.0,
-                                               lv == T.upper.nlevels - 1 && swap_out);
+#undef MPFFT_D_CASE
+  if (e != cudaSuccess) return e;
+  // The levels above: whole batches per launch.  (Groups of signals that fit
+  // L2 between the launches were slower at every size: 2^24 points, N = 8192
+  // 222 us, in groups of 2^21 points 282, 2^22 249, 2^23 240.)
+  const int lgN = 31 - __builtin_clz((unsigned)S.N), step = d_upper_levels(nl);
+  for (int done = 0; done < nl;) {
+    const int r = std::min(step, nl - done), lgu = S.lgT + done - 1, lgnch = lgN - (lgu + r + 1);
+    const bool last = done + r == nl;
+    const long long cols = (long long)B * (S.N >> (r + 1));
+    const unsigned blocks = (unsigned)((cols + 255) / 256);
+    const double sc = last ? scale : 1.0;
+    const int sw = last && swap_out;
+    if (r == 3) d_upper_kernel<3><<<blocks, 256, 0, s>>>(out, S.N, B, lgu, lgnch, S.tw, sc, sw);
+    else if (r == 2) d_upper_kernel<2><<<blocks, 256, 0, s>>>(out, S.N, B, lgu, lgnch, S.tw, sc, sw);
+    else d_upper_kernel<1><<<blocks, 256, 0, s>>>(out, S.N, B, lgu, lgnch, S.tw, sc, sw);
+    done += r;
   }
   return cudaGetLastError();
 }

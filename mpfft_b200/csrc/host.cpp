@@ -42,6 +42,7 @@
 #define MPFFT_MPFR_TYPES_PROVIDED 1
 #include "../../include/mpfft_b200.h"
 #include "mpfft_internal.h"
+#include "sr_chunks.cuh"
 
 #define MPFFT_API extern "C" __attribute__((visibility("default")))
 
@@ -594,7 +595,6 @@ struct mpfft_d_plan {
   double *d_wc = nullptr, *d_ws = nullptr;  // real plans: cos, sin of 2 pi k / n_real, k < N/2
   DeviceTree upper;                   // levels above the shared-memory sub-transforms
   std::vector<void *> dev_allocs;     // roots, perms, sub-schedule tables
-  double *d_wr = nullptr, *d_wi = nullptr;
   DDeviceTables tabs;
   cudaStream_t stream = nullptr;
   std::mutex mu;
@@ -605,8 +605,6 @@ struct mpfft_d_plan {
     if (scratch_ev) cudaEventDestroy(scratch_ev);
     for (cudaEvent_t e : piece_done) cudaEventDestroy(e);
     for (void *q : dev_allocs) cudaFree(q);
-    if (d_wr) cudaFree(d_wr);
-    if (d_wi) cudaFree(d_wi);
     if (d_in) cudaFree(d_in);
     if (d_out) cudaFree(d_out);
     if (h_in) cudaFreeHost(h_in);
@@ -1391,31 +1389,104 @@ static int build_sub(mpfft_d_plan *p, int size, SubSchedule &S, int leaf_max = 1
   return MPFFT_OK;
 }
 
-// sub_max: largest shared-memory sub-transform (0: the default kDSubMax; the
-// results do not depend on it, only where each butterfly runs)
+// Base cases of a T-point tree (T >= 32), one slot per 16 output positions,
+// ordered so that a warp's loads are of neighbouring input classes (16-point
+// leaves first) and its eight-lane shared-memory phases hit different banks
+// where the window of 32 slots allows it (key: the swizzled position's low 3
+// bits, d_swz in d_core.cuh).
+static std::vector<SrLeafSlot> leaf_slots(int T) {
+  HostTree t;
+  walk(t, T, 1, 0, 0, 16);
+  std::vector<SrLeafSlot> slots(T / 16);
+  for (const Leaf &lf : t.leaves) {
+    SrLeafSlot &s = slots[lf.out / 16];
+    s.m = lf.out / 16;
+    if (lf.out % 16 == 0) s.sna = lf.sn;
+    else s.snb = lf.sn;
+  }
+  auto cls = [&](const SrLeafSlot &s) { return ((s.sna % (T / 16)) + T / 16) % (T / 16); };
+  std::stable_sort(slots.begin(), slots.end(), [&](const SrLeafSlot &a, const SrLeafSlot &b) {
+    const bool ba = sr_chunk_big(a.m), bb = sr_chunk_big(b.m);
+    return ba != bb ? ba : cls(a) < cls(b);
+  });
+  std::vector<SrLeafSlot> out;
+  for (size_t w = 0; w < slots.size(); w += 32) {
+    const size_t e = std::min(slots.size(), w + 32);
+    for (int big = 1; big >= 0; --big) {
+      std::vector<SrLeafSlot> bank[8];
+      size_t left = 0;
+      for (size_t i = w; i < e; ++i)
+        if (sr_chunk_big(slots[i].m) == (big != 0)) {
+          const int m = 16 * slots[i].m;
+          bank[((m >> 3) ^ (m >> 6) ^ (m >> 9)) & 7].push_back(slots[i]);
+          ++left;
+        }
+      while (left) {  // one of each bank in turn, the fullest first
+        std::vector<int> order{0, 1, 2, 3, 4, 5, 6, 7};
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bank[a].size() > bank[b].size(); });
+        for (int k : order)
+          if (!bank[k].empty()) {
+            out.push_back(bank[k].front());
+            bank[k].erase(bank[k].begin());
+            --left;
+          }
+      }
+    }
+  }
+  return out;
+}
+
+// lg of the sub-transform size of an N-point FP64 transform longer than
+// kDSubMax: the smallest of 1024, 2048 and 4096 points that needs no more
+// passes of three levels above it than the others (smaller chunks let a CTA
+// hold several of neighbouring input classes).
+static int d_sub_lg(int lgN) {
+  int best = 12;
+  for (int l = 11; l >= 10; --l)
+    if ((lgN - l + 2) / 3 <= (lgN - best + 2) / 3) best = l;
+  return best;
+}
+
+// sub_max: shared-memory sub-transform size for transforms longer than it (0:
+// d_sub_lg; the results do not depend on it, only where each butterfly runs)
 static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
   if (!is_pow2(n)) return set_err(MPFFT_EINVAL, "n=%lu is not a power of two", n);
   if (n > (1UL << 28)) return set_err(MPFFT_EUNSUPPORTED, "n=%lu too large", n);
   if (int e = device_ready()) return e;
   p->N = n;
   p->tabs.N = (int)n;
-  // cut the tree at T points: maximal nodes of size <= T run in shared memory
-  const int T = (int)std::min<unsigned long>(n, sub_max > 0 ? sub_max : kDSubMax);
-  {
-    HostTree t;
-    walk(t, (int)n, 1, 0, 0, T);
-    std::vector<SubRoot> roots;
-    for (const Leaf &lf : t.leaves) roots.push_back(SubRoot{lf.sn, lf.s, lf.out, lf.n});
-    p->tabs.nroots = (int)roots.size();
-    if (int e = upload(p, roots, &p->tabs.roots)) return e;
-    if (int e = build_tree(p->upper, n, T)) return e;  // its levels are the ones above T
-    p->tabs.upper = p->upper.tabs;
+  DSubTab &S = p->tabs.d;
+  const int lgN = ilog2(n);
+  S.N = (int)n;
+  S.lgT = lgN;
+  if (sub_max > 0) {
+    int l = 10;
+    while (l < 12 && (2 << l) <= sub_max) ++l;
+    if (lgN > l) S.lgT = l;
+  } else if (n > (unsigned long)kDSubMax) {
+    S.lgT = d_sub_lg(lgN);
   }
-  if (int e = build_sub(p, T, p->tabs.sub[0])) return e;
-  if (T >= 2) {
-    if (int e = build_sub(p, T / 2, p->tabs.sub[1])) return e;
-  } else {
-    p->tabs.sub[1] = p->tabs.sub[0];
+  const int T = 1 << S.lgT;
+  S.nchunks = (int)(n / T);
+  if (n > 16) {
+    if (int e = upload(p, leaf_slots(T), &S.slots[0])) return e;
+    S.slots[1] = S.slots[0];
+    if (S.nchunks > 1) {
+      if (int e = upload(p, leaf_slots(T / 2), &S.slots[1])) return e;
+      HostTree t;
+      walk(t, (int)n, 1, 0, 0, T);
+      std::vector<SrChunk> chunks(S.nchunks);
+      for (const Leaf &lf : t.leaves) {
+        SrChunk &c = chunks[lf.out / T];
+        c.chunk = lf.out / T;
+        if (lf.out % T == 0) c.sna = lf.sn;
+        else c.snb = lf.sn;
+      }
+      auto cls = [&](const SrChunk &c) { return ((c.sna % S.nchunks) + S.nchunks) % S.nchunks; };
+      std::stable_sort(chunks.begin(), chunks.end(),
+                       [&](const SrChunk &a, const SrChunk &b) { return cls(a) < cls(b); });
+      if (int e = upload(p, chunks, &S.chunks)) return e;
+    }
   }
   // twiddles exactly as the reference lut() (serial_d_fft6.c:52-62)
   const unsigned long q = n / 4;
@@ -1424,18 +1495,26 @@ static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
     wr[k] = cos(2. * M_PI * k / n);
     wi[k] = sin(2. * M_PI * k / n);
   }
-  CUDA_TRY(cudaMalloc(&p->d_wr, wr.size() * sizeof(double)));
-  CUDA_TRY(cudaMalloc(&p->d_wi, wi.size() * sizeof(double)));
-  CUDA_TRY(cudaMemcpy(p->d_wr, wr.data(), wr.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CUDA_TRY(cudaMemcpy(p->d_wi, wi.data(), wi.size() * sizeof(double), cudaMemcpyHostToDevice));
-  p->tabs.wr = p->d_wr;
-  p->tabs.wi = p->d_wi;
-  p->tabs.c8 = cos(2. * M_PI * 1 / 8);
-  p->tabs.c16a = cos(2. * M_PI * 1 / 16);
-  p->tabs.c16b = cos(2. * M_PI * 1 / 16) - cos(2. * M_PI * 3 / 16);
-  p->tabs.c16c = cos(2. * M_PI * 3 / 16);
-  p->tabs.c16d = cos(2. * M_PI * 1 / 16) + cos(2. * M_PI * 3 / 16);
+  S.K.c8 = cos(2. * M_PI * 1 / 8);
+  S.K.c16a = cos(2. * M_PI * 1 / 16);
+  S.K.c16b = cos(2. * M_PI * 1 / 16) - cos(2. * M_PI * 3 / 16);
+  S.K.c16c = cos(2. * M_PI * 3 / 16);
+  S.K.c16d = cos(2. * M_PI * 1 / 16) + cos(2. * M_PI * 3 / 16);
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
+  if (n > 16) {  // the levels' twiddles, gathered from that table on the device
+    double *d_w = nullptr;
+    double2 *d_tw = nullptr;
+    CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2)));
+    p->dev_allocs.push_back(d_tw);
+    CUDA_TRY(cudaMalloc(&d_w, 2 * q * sizeof(double)));
+    cudaError_t e = cudaMemcpy(d_w, wr.data(), q * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d_w + q, wi.data(), q * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = d_build_level_tw(d_w, d_w + q, (int)n, d_tw, p->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+    cudaFree(d_w);
+    CUDA_TRY(e);
+    S.tw = d_tw;
+  }
   return MPFFT_OK;
 }
 

@@ -80,15 +80,42 @@ struct SubRoot {
   int sn, s, out, size;
 };
 
+// FP64 base-case constants
+struct DConst {
+  double c8 = 0, c16a = 0, c16b = 0, c16c = 0, c16d = 0;
+};
+
+// One thread's base cases of a sub-transform: the 16 output positions [16m,
+// 16m+16) hold a leaf of 16 points (input sna) or a pair of leaves of 8 points
+// (inputs sna, snb), in the sub-transform's own input sequence.
+struct SrLeafSlot {
+  int m, sna, snb;
+};
+// A chunk of T output positions of an N-point tree: one sub-transform of T
+// points (input sna, stride N/T) or a pair of T/2 points (sna, snb, 2N/T).
+struct SrChunk {
+  int chunk, sna, snb;
+};
+
+// FP64 plans (d_core.cuh): chunks of T = 2^lgT points run in shared memory
+struct DSubTab {
+  int N = 0, lgT = 0;
+  int nchunks = 0;                        // N/T
+  const SrLeafSlot *slots[2] = {};        // base cases of a T- and a T/2-point tree
+  const SrChunk *chunks = nullptr;        // by input class
+  const double2 *tw = nullptr;            // (cos, sin) per level, sr_level_tw
+  DConst K;
+};
+
 struct DDeviceTables {
   int N = 0;
+  DSubTab d;  // FP64 plans; the fields below: compensated tiers
   const double *wr = nullptr;  // [N/4] cos(2 pi k/N)
   const double *wi = nullptr;  // [N/4] sin(2 pi k/N)
   const double *wrl = nullptr, *wil = nullptr;  // double-double plans: low parts of wr, wi
   // compensated tiers (float_tier_kernels.cu): the words of cos and sin of
   // 2 pi k/N, k < N/4 (double-double: 2, quad-double: 4, float-float: 1 double)
   const double *tw_cos[4] = {}, *tw_sin[4] = {};
-  double c8 = 0, c16a = 0, c16b = 0, c16c = 0, c16d = 0;
   // shared-memory sub-transforms (sizes T and T/2) ...
   int nroots = 0;
   const SubRoot *roots = nullptr;
@@ -98,7 +125,8 @@ struct DDeviceTables {
 };
 
 constexpr int kMaxDevices = 64;
-constexpr int kDSubMax = 4096;  // FP64: largest shared-memory sub-transform (64 KB)
+constexpr int kDSubMax = 4096;  // FP64: most points a CTA holds in shared memory (64 KB)
+constexpr int kDSubMin = 64;    // FP64: smallest sub-transform of a longer transform
 constexpr int kDDSubMax = 2048; // double-double: largest shared-memory sub-transform (64 KB)
 constexpr int kQDSubMax = 1024; // quad-double (64 KB)
 constexpr int kFFSubMax = 4096; // float-float (64 KB)
@@ -209,6 +237,8 @@ cudaError_t mp_export_launch(const uint32_t *planes, int N, int B, int L, const 
 // out[m][c][r][e] = in[m][r][c][e]: nmat matrices of R x C elements of E words
 cudaError_t transpose_launch(const uint32_t *in, uint32_t *out, long long nmat, long long R, long long C, int E,
                              cudaStream_t s);
+// tw[sr_level_tw(n) + k] = (wr, wi)[k*(N/n)] for every level n = 32 .. N
+cudaError_t d_build_level_tw(const double *wr, const double *wi, int N, double2 *tw, cudaStream_t s);
 // FP64 layout: word (c, b, p) at base[(c*B + b)*N + p]  (signal-contiguous)
 // swap_in / swap_out: read the input's / write the output's real and imaginary
 // planes exchanged (both: the unscaled inverse, swap(FFT(swap(x))))

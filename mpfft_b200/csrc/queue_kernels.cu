@@ -63,35 +63,64 @@ __global__ void __launch_bounds__(256) mp_queue_kernel(const QueueItem *__restri
 }
 
 // ---------------------------------------------------------------------------
-// FP64: the sub-transform roots one after another in shared memory, then the
+// FP64: the chunks of T points one after another in shared memory, then the
 // levels above them in global memory
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) d_queue_kernel(const QueueItem *__restrict__ items, int nitems, int *head,
-                                                      double scale) {
-  extern __shared__ double dq_smem[];
+// one signal of N points: every chunk of T points, then the levels above
+template <int LGT>
+__device__ __forceinline__ void d_queue_signal(const DSubTab &S, DSubArgs A, double2 *sm) {
+  if (S.nchunks == 1) {
+    d_sub_transform<LGT, true>(S, A, sm);
+    return;
+  }
+  if constexpr (LGT >= 10) {
+    for (A.c0 = 0; A.c0 < S.nchunks; ++A.c0) {
+      __syncthreads();  // shared memory of the previous chunk is free
+      d_sub_transform<LGT, false>(S, A, sm);
+    }
+  }
+}
+
+template <int R>
+__device__ __forceinline__ void d_queue_upper(const DSubTab &S, double *out, int lgu, int cols, double scale) {
+  for (int t = threadIdx.x; t < cols; t += blockDim.x)
+    d_upper_column<R>(out, S.N, 1, lgu, 0, t >> lgu, t & ((1 << lgu) - 1), S.tw, scale, false);
+}
+
+__global__ void __launch_bounds__(256, 2) d_queue_kernel(const QueueItem *__restrict__ items, int nitems, int *head,
+                                                         double scale) {
+  extern __shared__ __align__(16) double2 dq_smem[];
   __shared__ int slot;
   for (int i; (i = queue_next(head, &slot)) < nitems;) {
     const QueueItem it = items[i];
-    const DDeviceTables &T = it.tab->ft;
-    const double *in = static_cast<const double *>(it.in);
+    const DSubTab S = it.tab->ft.d;
     double *out = static_cast<double *>(it.out);
-    const DConst K{T.c8, T.c16a, T.c16b, T.c16c, T.c16d};
-    const bool final_sub = T.upper.nlevels == 0;
-    for (int r = 0; r < T.nroots; ++r) {
-      __syncthreads();  // shared memory of the previous root is free
-      d_sub_instances<false>(in, out, T.N, 1, 0, 1, T.roots[r], T.sub[0], T.sub[1], T.wr, T.wi, K,
-                             final_sub ? scale : 1.0, 0, 0, dq_smem);
+    const int nl = S.N > 16 ? 31 - __clz(S.nchunks) : 0;
+    const DSubArgs A{static_cast<const double *>(it.in), out, 1, 0, 0, 1, scale, nl == 0, false, false};
+    if (S.N <= 16) {
+      d_tiny(S, A, dq_smem);
+      continue;
     }
-    for (int lv = 0; lv < T.upper.nlevels; ++lv) {
+    switch (S.lgT) {
+      case 5: d_queue_signal<5>(S, A, dq_smem); break;
+      case 6: d_queue_signal<6>(S, A, dq_smem); break;
+      case 7: d_queue_signal<7>(S, A, dq_smem); break;
+      case 8: d_queue_signal<8>(S, A, dq_smem); break;
+      case 9: d_queue_signal<9>(S, A, dq_smem); break;
+      case 10: d_queue_signal<10>(S, A, dq_smem); break;
+      case 11: d_queue_signal<11>(S, A, dq_smem); break;
+      case 12: d_queue_signal<12>(S, A, dq_smem); break;
+      default: break;
+    }
+    const int step = d_upper_levels(nl);
+    for (int done = 0; done < nl;) {
       __syncthreads();
-      const int n = T.upper.level_n[lv], q = n >> 2;
-      const int total = T.upper.level_count[lv] * q;
-      const int *nodes = T.upper.node_off + T.upper.level_start[lv];
-      const double sc = lv == T.upper.nlevels - 1 ? scale : 1.0;
-      for (int t = threadIdx.x; t < total; t += blockDim.x) {
-        const int k = t % q, kn = k * (T.N / n);
-        d_butterfly(out, out + T.N, 1, nodes[t / q], k, q, T.wr[kn], T.wi[kn], sc, false);
-      }
+      const int r = min(step, nl - done), lgu = S.lgT + done - 1, cols = S.N >> (r + 1);
+      const double sc = done + r == nl ? scale : 1.0;
+      if (r == 3) d_queue_upper<3>(S, out, lgu, cols, sc);
+      else if (r == 2) d_queue_upper<2>(S, out, lgu, cols, sc);
+      else d_queue_upper<1>(S, out, lgu, cols, sc);
+      done += r;
     }
   }
 }

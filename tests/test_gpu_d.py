@@ -98,3 +98,33 @@ def test_d_inverse_bitexact_vs_reference_procedure(M, orc, n):
     zr, zi = np.zeros(n), np.zeros(n)
     plan.execute(1, xr, xi, zr, zi, scaled=True, inverse=True)
     assert _bits_equal(zr, er) and _bits_equal(zi, ei)
+
+
+@pytest.mark.parametrize("n,batch", [(8, 700), (16, 129), (32, 333), (64, 65), (128, 33), (256, 301), (512, 9),
+                                     (1024, 5), (2048, 3), (4096, 2), (8192, 3), (16384, 2), (32768, 1), (131072, 1),
+                                     (1 << 19, 1)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_d_register_passes_bitexact(M, orc, n, batch, inverse):
+    """Every chain of base cases and register passes (up to three levels each,
+    in shared memory and above), CTAs of several signals with a partly filled
+    last one, planes exchanged and scaled outputs: the same bits as the
+    reference's transform (inverse: its swap procedure, lab/serial/double/
+    serial_d_fft6.c:511-524)."""
+    import torch
+
+    rng = np.random.default_rng(n + batch)
+    x = rng.uniform(-1, 1, (2, batch, n))
+    d_in = torch.from_numpy(x).cuda()
+    d_out = torch.full_like(d_in, float("nan"))
+    plan = M.DPlan(n)
+    plan.execute_device(batch, d_in.data_ptr(), d_out.data_ptr(), scaled=inverse, inverse=inverse,
+                        stream=torch.cuda.current_stream().cuda_stream)
+    y = d_out.cpu().numpy()
+    f = orc.DFFT(n)
+    for b in sorted({0, batch // 2, batch - 1}):
+        if inverse:
+            ei, er = f(x[1, b].copy(), x[0, b].copy())
+            er, ei = er / n, ei / n
+        else:
+            er, ei = f(x[0, b].copy(), x[1, b].copy())
+        assert _bits_equal(y[0, b], er) and _bits_equal(y[1, b], ei), b
