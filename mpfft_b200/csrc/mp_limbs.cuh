@@ -56,6 +56,38 @@ __device__ __forceinline__ uint32_t addc(uint32_t a, uint32_t b, uint32_t &c) {
   return (uint32_t)t;
 }
 
+// Carry chains through the condition code: cc_set(c) sets the carry flag to c
+// (0 or 1), add_cc / addc_cc add and set it, carry() reads it.  One chain at a time, with
+// nothing else between its steps; the steps are volatile, so they stay in
+// program order.  (One instruction per limb; addc above takes two.)
+__device__ __forceinline__ void cc_set(uint32_t c) {
+  uint32_t t;
+  asm volatile("add.cc.u32 %0, %1, 0xffffffff;" : "=r"(t) : "r"(c));
+}
+__device__ __forceinline__ uint32_t add_cc(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t addc_cc(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm volatile("addc.cc.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t carry() {
+  uint32_t r;
+  asm volatile("addc.u32 %0, 0, 0;" : "=r"(r));
+  return r;
+}
+// (hi:lo) += x * t, carry out (mad_cc), carry in and out (madc_cc): the two
+// halves of one product side by side, which is one 32x32+64-bit multiply-add
+__device__ __forceinline__ void mad_cc(uint32_t &lo, uint32_t &hi, uint32_t x, uint32_t t) {
+  asm volatile("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(x), "r"(t));
+}
+__device__ __forceinline__ void madc_cc(uint32_t &lo, uint32_t &hi, uint32_t x, uint32_t t) {
+  asm volatile("madc.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.cc.u32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(x), "r"(t));
+}
+
 template <int L>
 __device__ __forceinline__ void ld(uint32_t (&x)[L], const uint32_t *p, size_t plane) {
 #pragma unroll
@@ -77,9 +109,15 @@ __device__ __forceinline__ void ld_addsub(uint32_t (&x)[L], const uint32_t *pa, 
     return;
   }
   const uint32_t m = subtract ? 0xffffffffu : 0u;
-  uint32_t c = subtract ? 1u : 0u;
+  uint32_t y[L];
 #pragma unroll
-  for (int i = 0; i < L; ++i, pa += plane, pb += plane) x[i] = addc(*pa, *pb ^ m, c);
+  for (int i = 0; i < L; ++i, pa += plane, pb += plane) {
+    x[i] = *pa;
+    y[i] = *pb ^ m;
+  }
+  cc_set(subtract ? 1u : 0u);
+#pragma unroll
+  for (int i = 0; i < L; ++i) x[i] = addc_cc(x[i], y[i]);
 }
 
 // x = sx*x + sp*p with sx in {+1,-1}, sp in {+1,-1,0}; p streamed from memory.
@@ -90,9 +128,12 @@ __device__ __forceinline__ void combine_p(uint32_t (&x)[L], const uint32_t *p, s
   const uint32_t mx = negx ? 0xffffffffu : 0u;
   const uint32_t mp = sp < 0 ? 0xffffffffu : 0u;
   const uint32_t keep = sp != 0 ? 0xffffffffu : 0u;
-  uint32_t c = (negx ? 1u : 0u) + (sp < 0 ? 1u : 0u);
+  uint32_t y[L];
 #pragma unroll
-  for (int i = 0; i < L; ++i, p += stride) x[i] = addc(x[i] ^ mx, (*p & keep) ^ mp, c);
+  for (int i = 0; i < L; ++i, p += stride) y[i] = (*p & keep) ^ mp;
+  cc_set(negx || sp < 0 ? 1u : 0u);
+#pragma unroll
+  for (int i = 0; i < L; ++i) x[i] = addc_cc(x[i] ^ mx, y[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -110,10 +151,15 @@ __device__ __forceinline__ void combine_p(uint32_t (&x)[L], const uint32_t *p, s
 // place.  Adding 2^(32L-2) before the final shift rounds to nearest.
 //
 // The product is formed row by row (operand scanning): for each twiddle limb
-// w_j, one multiply-add-carry chain adds x_i*w_j into columns i+j.  Each step
-// is a 32x32+32+32 -> 64-bit multiply-add (it cannot overflow), written in
-// plain C so the compiler can schedule the two halves freely; on sm_100a this
-// issues faster than PTX mad.lo.cc/madc.hi.cc chains (measured).
+// w_j the products x_i*w_j go to columns i+j and i+j+1.  Two accumulators,
+// one for products whose low half falls on an even column (counted from L-2)
+// and one for the odd ones, so that the products of a row fall on disjoint
+// column pairs of each and run as two carry chains of one 32x32+64-bit
+// multiply-add per product (mad_cc / madc_cc); the accumulators are added once
+// at the end.  A form that adds each product's halves and a carry in C takes
+// three instructions per product; the products are bound by instruction issue,
+// so that costs (N=1024, batch 2048, us per batch, that form / this one): 9
+// limbs 470 / 432, 17 limbs 1057 / 907, 25 limbs 1810 / 1521, 33 limbs 2810 / 2330.
 //
 // kPacked: w holds the L limbs contiguously in shared memory, 16-byte aligned
 // (tplane unused); they are read four at a time with 128-bit loads.
@@ -129,32 +175,47 @@ __device__ __forceinline__ void mul_tw(uint32_t (&x)[L], const uint32_t *w, size
   };
   const uint32_t smask = 0u - (x[L - 1] >> 31);
 
-  // acc[a] holds column (L-2+a), a = 0 .. L+1
-  uint32_t acc[L + 2];
+  // ev[a] + od[a] is column (L-2+a), a = 0 .. L+1; ev holds the products with
+  // even a in the pairs (a, a+1), od those with odd a
+  uint32_t ev[L + 4], od[L + 4];
 #pragma unroll
-  for (int a = 0; a < L + 2; ++a) acc[a] = 0;
-  acc[1] = 1u << 30;  // + 2^(32L-2): round to nearest on the final >> (32L-1)
+  for (int a = 0; a < L + 4; ++a) ev[a] = od[a] = 0;
+  ev[1] = 1u << 30;  // + 2^(32L-2): round to nearest on the final >> (32L-1)
 
   const uint32_t *w0 = w;
 #pragma unroll
   for (int j = 0; j < L; ++j, w += kPacked ? 0 : tplane) {
     const uint32_t t = limb(w, j);
     const int i0 = (L - 2 - j) > 0 ? (L - 2 - j) : 0;
-    uint32_t c = 0;
+    // rows below j reach column j+1, so the chains' carries land on empty words
 #pragma unroll
-    for (int i = i0; i < L; ++i) {
-      const uint64_t pr = (uint64_t)x[i] * t + acc[i + j - (L - 2)] + c;
-      acc[i + j - (L - 2)] = (uint32_t)pr;
-      c = (uint32_t)(pr >> 32);
+    for (int par = 0; par < 2; ++par) {
+      uint32_t(&acc)[L + 4] = par ? od : ev;
+      const int a0 = i0 + j - (L - 2);
+      const int first = i0 + ((a0 & 1) != par ? 1 : 0);
+      if (first < L) {
+        int a = 0;
+#pragma unroll
+        for (int i = first; i < L; i += 2) {
+          a = i + j - (L - 2);
+          if (i == first) mad_cc(acc[a], acc[a + 1], x[i], t);
+          else madc_cc(acc[a], acc[a + 1], x[i], t);
+        }
+        if (a + 2 <= L + 1) acc[a + 2] = carry();
+      }
     }
-    acc[j + 2] = c;  // column L+j is still empty: rows < j reach column L+j-1
   }
-  // signed correction: acc -= s * w * 2^(32L)  (columns L .. 2L-1 = acc[2 .. L+1])
-  {
-    uint32_t c = 1;
+  // columns = ev + od, minus s * w * 2^(32L) (columns L .. 2L-1, a = 2 .. L+1)
+  uint32_t acc[L + 2];
+  acc[0] = add_cc(ev[0], od[0]);
 #pragma unroll
-    for (int j = 0; j < L; ++j, w0 += kPacked ? 0 : tplane) acc[j + 2] = addc(acc[j + 2], ~(limb(w0, j) & smask), c);
-  }
+  for (int a = 1; a < L + 2; ++a) acc[a] = addc_cc(ev[a], od[a]);
+  uint32_t nw[L];
+#pragma unroll
+  for (int j = 0; j < L; ++j, w0 += kPacked ? 0 : tplane) nw[j] = ~(limb(w0, j) & smask);
+  cc_set(1u);
+#pragma unroll
+  for (int j = 0; j < L; ++j) acc[j + 2] = addc_cc(acc[j + 2], nw[j]);
   // x = (columns L-1 .. 2L-1) >> 31
 #pragma unroll
   for (int i = 0; i < L; ++i) x[i] = __funnelshift_r(acc[i + 1], acc[i + 2], 31);
