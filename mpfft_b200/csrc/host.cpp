@@ -416,9 +416,11 @@ static int mp_limbs_for(unsigned long N, long P) {
 
 struct MpTwiddles {
   uint32_t *d_tw = nullptr;
+  uint32_t *d_twp = nullptr;  // packed copy (mp_pack_tw), up to kMaxLimbs limbs
   uint8_t *d_dneg = nullptr;
   ~MpTwiddles() {
     if (d_tw) cudaFree(d_tw);
+    if (d_twp) cudaFree(d_twp);
     if (d_dneg) cudaFree(d_dneg);
   }
 };
@@ -679,6 +681,12 @@ static int mp_plan_init(mpfft_mp_plan *p, unsigned long n, long prec, bool host_
   p->tabs.dneg = p->tw.d_dneg;
   p->tabs.tws = real ? 2 : 1;
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
+  if (L <= kMaxLimbs && nt >= 16) {
+    CUDA_TRY(cudaMalloc(&p->tw.d_twp, mp_packed_tw_words(L, (long long)n / 4) * sizeof(uint32_t)));
+    CUDA_TRY(mp_pack_tw(p->tw.d_tw, p->tw.d_twp, L, (long long)n / 4, p->stream));
+    CUDA_TRY(cudaStreamSynchronize(p->stream));
+    p->tabs.twp = p->tw.d_twp;
+  }
   return MPFFT_OK;
 }
 

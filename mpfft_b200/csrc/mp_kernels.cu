@@ -745,6 +745,8 @@ cudaError_t mp_run_transform(int L, const MpDeviceTables &T, const uint32_t *in,
     if ((!big_scratch && T.nlevels > 0) || L > kMaxLimbsBig) return cudaErrorInvalidValue;
     return mp_big_run_transform(L, T, in, out, B, big_scratch, s, launch_ms);
   }
+  // (timed calls run level by level, so that the time can be told by level)
+  if (!launch_ms && mp_tile_used(T, L, B)) return mp_tile_run(L, T, in, out, B, s);
   switch (L) {
     MPFFT_MP_CASE(2) MPFFT_MP_CASE(3) MPFFT_MP_CASE(4) MPFFT_MP_CASE(5) MPFFT_MP_CASE(6) MPFFT_MP_CASE(7)
     MPFFT_MP_CASE(8) MPFFT_MP_CASE(9) MPFFT_MP_CASE(10) MPFFT_MP_CASE(11) MPFFT_MP_CASE(12)

@@ -47,6 +47,7 @@ struct MpDeviceTables : TreeTables {
   const uint32_t *tw = nullptr;   // [3][L][tws*N/4]: cos, cos+sin, |cos-sin| magnitudes
   const uint8_t *dneg = nullptr;  // [tws*N/4]: sign of cos-sin
   int tws = 1;  // the table is built for tws*N points (2 for a real transform of 2N points)
+  const uint32_t *twp = nullptr;  // [tws*N/4][3][L rounded up to 4]: the same, one twiddle's limbs together
   int tc = 1;   // twiddle products on the tensor cores (mp_tc_kernels.cu): 0 never, 1 from
                 // kTcMinLimbs limbs, 2 from kTcForceMinLimbs limbs
 };
@@ -198,6 +199,11 @@ struct LaunchTimer {
 // (and only used) when L > kMaxLimbs.
 cudaError_t mp_run_transform(int L, const MpDeviceTables &T, const uint32_t *in, uint32_t *out, int B,
                              cudaStream_t s, float *launch_ms = nullptr, uint32_t *big_scratch = nullptr);
+// several levels per launch in shared memory (mp_smem_kernels.cu), L <= kMaxLimbs
+bool mp_tile_used(const MpDeviceTables &T, int L, int B);
+cudaError_t mp_tile_run(int L, const MpDeviceTables &T, const uint32_t *in, uint32_t *out, int B, cudaStream_t s);
+size_t mp_packed_tw_words(int L, long long n4);
+cudaError_t mp_pack_tw(const uint32_t *tw, uint32_t *twp, int L, long long n4, cudaStream_t s);
 size_t mp_big_scratch_words(const MpDeviceTables &T, int L, int B);
 cudaError_t mp_big_run_transform(int L, const MpDeviceTables &T, const uint32_t *in, uint32_t *out, int B,
                                  uint32_t *scratch, cudaStream_t s, float *launch_ms);

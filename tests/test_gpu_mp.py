@@ -399,3 +399,30 @@ def test_mp_large_precision(M, orc, n, p, batch):
         O.MpFFT(n, p)(sr, si, rr, ri)
         e_ref = O.mp_errors(rr, ri, dr, di)["log2_rel"]
         assert e_gpu <= O.mp_bound_log2(n, p) and e_gpu <= e_ref + 0.5, (e_gpu, e_ref)
+
+
+@pytest.mark.parametrize("n,p,B", [(16, 30, 700), (16, 60, 4096), (32, 120, 301), (64, 53, 137), (128, 250, 100),
+                                   (256, 330, 97), (512, 380, 65), (1024, 256, 13), (1024, 400, 53), (2048, 100, 5),
+                                   (2048, 430, 25), (4096, 64, 3), (4096, 600, 13), (1024, 600, 64), (512, 800, 128),
+                                   (256, 1000, 200), (1024, 1024, 49), (16384, 256, 1), (8192, 512, 7)])
+def test_mp_tiles_bit_identical(M, n, p, B):
+    """Batches whose levels run several per launch in shared-memory tiles: full
+    and partly filled signal groups, chunks that are one node and pairs, one to
+    three launches.  Single signals cut from the batch run level by level (timed
+    call): the outputs are bit-identical."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    plan = M.MpPlan(n, p)
+    L = plan.limbs
+    host = synthetic_planes(n, L, plan.frac_bits, B, seed=n + B).reshape(2, L, n, B)
+    s = torch.cuda.current_stream().cuda_stream
+    d_in = torch.from_numpy(np.ascontiguousarray(host).view(np.int32)).cuda()
+    d_out = torch.full_like(d_in, -1)
+    plan.execute_device(B, d_in.data_ptr(), d_out.data_ptr(), s)
+    for b in sorted({0, B // 2, B - 1}):
+        one = d_in[..., b].contiguous()
+        ref = torch.empty_like(one)
+        plan.execute_device_timed(1, one.data_ptr(), ref.data_ptr(), s)
+        assert torch.equal(d_out[..., b].contiguous(), ref), b
