@@ -1510,17 +1510,15 @@ static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
   S.K.c16d = cos(2. * M_PI * 1 / 16) + cos(2. * M_PI * 3 / 16);
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
   if (n > 16) {  // the levels' twiddles, gathered from that table on the device
-    double *d_w = nullptr;
+    // (one allocation, the source table behind the levels: freeing it here would synchronise the device)
     double2 *d_tw = nullptr;
-    CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2)));
+    CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2) + 2 * q * sizeof(double)));
     p->dev_allocs.push_back(d_tw);
-    CUDA_TRY(cudaMalloc(&d_w, 2 * q * sizeof(double)));
-    cudaError_t e = cudaMemcpy(d_w, wr.data(), q * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_w + q, wi.data(), q * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = d_build_level_tw(d_w, d_w + q, (int)n, d_tw, p->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
-    cudaFree(d_w);
-    CUDA_TRY(e);
+    double *d_w = reinterpret_cast<double *>(d_tw + (n / 2 - 8));
+    CUDA_TRY(cudaMemcpyAsync(d_w, wr.data(), q * sizeof(double), cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_w + q, wi.data(), q * sizeof(double), cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(d_build_level_tw(d_w, d_w + q, (int)n, d_tw, p->stream));
+    CUDA_TRY(cudaStreamSynchronize(p->stream));
     S.tw = d_tw;
   }
   return MPFFT_OK;

@@ -117,7 +117,64 @@ __global__ void __launch_bounds__(256) mp_big_leaf_kernel(const uint32_t *__rest
   uint32_t *y = out + (size_t)lf.out * B + b;
   const size_t yB = B;
   int64_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int i = 0; i < L; ++i) {
+  // blocks of limbs whose 32 loads are in flight together (limb by limb the
+  // kernel waited out one memory latency per limb), then the last limbs
+  int i = 0;
+  if (lf.n == 4) {
+    constexpr int kU = 4;
+    for (; i + kU < L; i += kU) {
+      uint32_t vr[kU][4], vi[kU][4];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          vr[u][j] = x[j][(size_t)(i + u) * plane];
+          vi[u][j] = x[j][(size_t)(i + u) * plane + cim];
+        }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const size_t o = (size_t)(i + u) * plane;
+        const int64_t r0 = vr[u][0], r1 = vr[u][1], r2 = vr[u][2], r3 = vr[u][3];
+        const int64_t m0 = vi[u][0], m1 = vi[u][1], m2 = vi[u][2], m3 = vi[u][3];
+        const int64_t v[8] = {c[0] + r0 + r2 + r1 + r3, c[1] + r0 - r2 + m1 - m3, c[2] + r0 + r2 - r1 - r3,
+                              c[3] + r0 - r2 - m1 + m3, c[4] + m0 + m2 + m1 + m3, c[5] + m0 - m2 - r1 + r3,
+                              c[6] + m0 + m2 - m1 - m3, c[7] + m0 - m2 + r1 - r3};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          y[o + q * yB] = (uint32_t)v[q];
+          y[o + cim + q * yB] = (uint32_t)v[4 + q];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) c[q] = v[q] >> 32;
+      }
+    }
+  } else if (lf.n == 2) {
+    constexpr int kU = 8;
+    for (; i + kU < L; i += kU) {
+      uint32_t a[kU][4];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const size_t o = (size_t)(i + u) * plane;
+        a[u][0] = x[0][o];
+        a[u][1] = x[1][o];
+        a[u][2] = x[0][o + cim];
+        a[u][3] = x[1][o + cim];
+      }
+#pragma unroll
+      for (int u = 0; u < kU; ++u) {
+        const size_t o = (size_t)(i + u) * plane;
+        const int64_t r0 = a[u][0], r1 = a[u][1], m0 = a[u][2], m1 = a[u][3];
+        const int64_t v[4] = {c[0] + r0 + r1, c[1] + r0 - r1, c[2] + m0 + m1, c[3] + m0 - m1};
+        y[o] = (uint32_t)v[0];
+        y[o + yB] = (uint32_t)v[1];
+        y[o + cim] = (uint32_t)v[2];
+        y[o + cim + yB] = (uint32_t)v[3];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) c[q] = v[q] >> 32;
+      }
+    }
+  }
+  for (; i < L; ++i) {
     const size_t o = (size_t)i * plane;
     const bool top = i == L - 1;
     auto s64 = [top](uint32_t v) -> int64_t { return top ? (int64_t)(int32_t)v : (int64_t)v; };
@@ -234,15 +291,13 @@ __global__ void __launch_bounds__(128) mp_big_level_kernel(uint32_t *__restrict_
 }
 
 size_t mp_big_scratch_words(const MpDeviceTables &T, int L, int B) {
+  if (mp_tc_used(T, L)) return mp_tc_scratch_words(T, L, B);
   long long most = 0;
   for (int lv = 0; lv < T.nlevels; ++lv) {
     const long long th = (long long)T.level_count[lv] * (T.level_n[lv] / 4) * B;
     if (th > most) most = th;
   }
-  const size_t words = (size_t)2 * L * (size_t)most;
-  if (!mp_tc_used(T, L)) return words;
-  const size_t tcw = mp_tc_scratch_words(T, L, B);
-  return tcw > words ? tcw : words;
+  return (size_t)2 * L * (size_t)most;
 }
 
 cudaError_t mp_big_run_transform(int L, const MpDeviceTables &T, const uint32_t *in, uint32_t *out, int B,

@@ -116,3 +116,45 @@ def _slice(O, a, start, count, prec):
     out = O.MpArray(count, prec)
     O.lib().orc_mp_copy(out.ptr, a.ptr + start * MPFR_T, count)
     return out
+
+
+@pytest.mark.parametrize("n,p,B", [(8, 1100, 1), (16, 1300, 130), (64, 1070, 257), (128, 2100, 3), (256, 4200, 129),
+                                   (1024, 1600, 2), (512, 8100, 1)])
+def test_tc_items_match_one_launch_per_level(M, n, p, B):
+    """The persistent launch, whose items wait for the three items they need,
+    against one launch per level (the timed call): the same bits, for one and
+    several signal groups and every level order from one level up."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    plan = M.MpPlan(n, p)
+    host = synthetic_planes(n, plan.limbs, plan.frac_bits, B, seed=n + B)
+    s = torch.cuda.current_stream().cuda_stream
+    d_in = torch.from_numpy(host.view(np.int32)).cuda()
+    a, b = torch.full_like(d_in, -1), torch.full_like(d_in, -1)
+    for _ in range(3):
+        plan.execute_device(B, d_in.data_ptr(), a.data_ptr(), s)
+        plan.execute_device_timed(B, d_in.data_ptr(), b.data_ptr(), s)
+        assert torch.equal(a, b)
+    M.tc_error()
+
+
+def test_tc_segment_carries(M):
+    """Operands whose carries and signs run through whole segments: zeros,
+    powers of two, all ones, one limb of ones between zeros."""
+    import torch
+
+    for L in (35, 36, 41, 64, 129, 257):
+        full = (1 << (32 * L - 2)) - 1
+        xs = [0, 1, -1, full, -full, 1 << (16 * L), -(1 << (16 * L)), (1 << (16 * L)) - 1, -((1 << (16 * L)) - 1),
+              0xFFFFFFFF << 64, -(0xFFFFFFFF << 64), full ^ 0xFFFFFFFF, -(full ^ ((1 << (32 * (L // 2))) - 1))]
+        for w in ((1 << (32 * L)) - 1, 1 << (32 * L - 1), (1 << (32 * L - 1)) - 1):
+            x = torch.from_numpy(_to_planes(xs, L).view(np.int32)).cuda()
+            d_w = torch.from_numpy(_to_planes([w], L).view(np.int32)).cuda()
+            y = torch.zeros_like(x)
+            M.tc_mul(L, len(xs), x.data_ptr(), d_w.data_ptr(), y.data_ptr(),
+                     torch.cuda.current_stream().cuda_stream)
+            got = _from_planes(y.cpu().numpy().view(np.uint32))
+            for v, g in zip(xs, got):
+                assert g == _tc_expected(v, w, L), (L, hex(v)[:20], hex(w)[:20])
