@@ -8,86 +8,131 @@
 
 namespace mpfft {
 
+// Two CTAs of 256 threads per SM, 128 registers.  Measured (4096 points x 512,
+// us): double-double with two levels per pass 139, one 145, two at 85 registers
+// 160; quad-double with one level per pass 582, with 192 threads 631, three CTAs
+// of 192 (spilling) 686, two levels per pass (8 points, 255 registers) 896.  One
+// CTA of 512 threads with a chunk twice as large, which saves a pass above:
+// double-double 152, quad-double 617.
 template <class NT, bool SINGLE>
-__global__ void __launch_bounds__(256) tier_sub_kernel(const typename NT::W *__restrict__ in,
-                                                       typename NT::W *__restrict__ out, int N, int B,
-                                                       const SubRoot *__restrict__ roots, int nroots, int G,
-                                                       SubSchedule big, SubSchedule small, TierTw tw, double scale,
-                                                       int swap_in, int swap_out) {
-  extern __shared__ __align__(16) unsigned char tier_smem[];
-  typename NT::W *sm = reinterpret_cast<typename NT::W *>(tier_smem);
+__global__ void __launch_bounds__(256, 2)
+    tier_sub_kernel(const __grid_constant__ TierTab S, TierArgs<NT> A, int groups) {
+  extern __shared__ __align__(16) double2 tier_smem[];
+  const int g = A.G;
   if (SINGLE) {
-    const int b0 = blockIdx.x * G;
-    tier_sub_instances<NT, true>(in, out, N, B, b0, min(G, B - b0), roots[0], big, small, tw, scale, swap_in, swap_out,
-                                 sm);
+    A.b0 = blockIdx.x * g;
+    A.G = min(g, A.B - A.b0);
   } else {
-    tier_sub_instances<NT, false>(in, out, N, B, blockIdx.x / nroots, 1, roots[blockIdx.x % nroots], big, small, tw,
-                                  scale, swap_in, swap_out, sm);
+    A.b0 = blockIdx.x / groups;
+    A.c0 = (blockIdx.x % groups) * g;
+    A.G = min(g, S.nchunks - A.c0);
   }
+  tier_sub_transform<NT, SINGLE>(S, A, tier_smem);
 }
 
 template <class NT>
-__global__ void __launch_bounds__(256) tier_level_kernel(typename NT::W *__restrict__ y, int N, int B, int n,
-                                                         const int *__restrict__ node_off, int nnodes, TierTw tw,
+__global__ void __launch_bounds__(256) tier_tiny_kernel(const __grid_constant__ TierTab S, TierArgs<NT> A) {
+  A.b0 = blockIdx.x * A.G;
+  A.G = min(A.G, A.B - A.b0);
+  tier_tiny<NT>(S, A);
+}
+
+template <class NT, int R>
+__global__ void __launch_bounds__(256) tier_upper_kernel(typename NT::W *__restrict__ y,
+                                                         const __grid_constant__ TierTab S, int B, int lgu, int lgnch,
                                                          double scale, int swap_out) {
-  const int q = n >> 2;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nnodes * q * B) return;
-  const long long r = t / q;
-  tier_level_one<NT>(y, N, B, n, node_off[(int)(r % nnodes)], (int)(t % q), (int)(r / nnodes), tw, scale, swap_out);
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long r = e >> lgu;
+  const long long b = r >> lgnch;
+  if (b >= B) return;
+  tier_upper_column<NT, R>(y, S, B, lgu, (int)b, (int)(r & ((1 << lgnch) - 1)), (int)(e & ((1 << lgu) - 1)), scale,
+                           swap_out != 0);
 }
 
-constexpr size_t kTierSmemBytes = 64 * 1024;  // planes of one CTA
+__global__ void __launch_bounds__(256) tier_tw_kernel(const double *__restrict__ w, int words, int N,
+                                                      double2 *__restrict__ tw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of a plane
+  const int len = N / 2 - 2;
+  if (i >= len) return;
+  const int q = 1 << (31 - __clz(i + 2));  // n/4 of its level: entries q-2 .. 2q-3
+  const size_t kn = (size_t)(i + 2 - q) * (N / (4 * q)), n4 = (size_t)N / 4;
+  for (int h = 0; h < words; ++h)
+    tw[(size_t)h * len + i] = make_double2(w[(size_t)(2 * h) * n4 + kn], w[(size_t)(2 * h + 1) * n4 + kn]);
+}
+
+cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaStream_t s) {
+  tier_tw_kernel<<<(N / 2 + 255) / 256, 256, 0, s>>>(w, words, N, tw);
+  return cudaGetLastError();
+}
+
+template <class NT, bool SINGLE>
+static cudaError_t tier_sub_launch(const TierTab &S, TierArgs<NT> A, cudaStream_t s) {
+  // chunks per CTA: as many as fit, but no more than leave two CTAs for every SM
+  const long long inst = SINGLE ? A.B : (long long)S.nchunks * A.B;
+  int g = 1 << (NT::kLgMax - S.lgT);
+  while (g > 1 && inst / g < 2 * 148) g /= 2;
+  A.G = g;
+  // few CTAs: one level per pass, so that each pass has the most threads (one
+  // 1024-point float-float signal: 14.4 us with three levels per pass)
+  A.per = inst / g < 148 ? 1 : NT::kLevels;
+  const size_t smem = ((size_t)g << S.lgT) * NT::kUnits * sizeof(double2) + kOrderBytes;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(tier_sub_kernel<NT, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (NT::kUnits << NT::kLgMax) * (int)sizeof(double2) + (int)kOrderBytes);
+    if (e != cudaSuccess) return e;
+  }
+  const int threads = std::min(256, std::max(32, (g << S.lgT) >> (A.per + 1)));
+  const int groups = SINGLE ? 1 : (S.nchunks + g - 1) / g;
+  const long long ctas = SINGLE ? ((long long)A.B + g - 1) / g : (long long)groups * A.B;
+  tier_sub_kernel<NT, SINGLE><<<(unsigned)ctas, threads, smem, s>>>(S, A, groups);
+  return cudaGetLastError();
+}
 
 template <class NT>
-static cudaError_t tier_run(const DDeviceTables &T, const void *in_, void *out_, int B, double scale, cudaStream_t s,
+static cudaError_t tier_run(const DDeviceTables &T, const void *in, void *out, int B, double scale, cudaStream_t s,
                             bool swap_in, bool swap_out) {
   using W = typename NT::W;
-  const W *in = static_cast<const W *>(in_);
-  W *out = static_cast<W *>(out_);
-  const int size = T.sub[0].size;
-  const size_t inst_bytes = (size_t)2 * NT::K * size * sizeof(W);
-  const int G = T.nroots != 1 ? 1 : (int)std::max<size_t>(1, kTierSmemBytes / inst_bytes);
-  const size_t smem = (size_t)G * inst_bytes;
-  static bool attr_set = false;  // idempotent; benign race
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tier_sub_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kTierSmemBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(tier_sub_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kTierSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
+  const TierTab &S = T.t;
+  const int nl = 31 - __builtin_clz((unsigned)S.nchunks);  // levels above the sub-transforms
+  TierArgs<NT> A{static_cast<const W *>(in), static_cast<W *>(out), B, 0, 0, 0, NT::kLevels, scale, nl == 0, swap_in,
+                 swap_out && nl == 0};
+  if (S.N < 8) {
+    A.G = 256;
+    tier_tiny_kernel<NT><<<(unsigned)((B + 255) / 256), 256, 0, s>>>(S, A);
+    return cudaGetLastError();
   }
-  TierTw tw{};
-  for (int h = 0; h < 4; ++h) {
-    tw.c[h] = T.tw_cos[h];
-    tw.s[h] = T.tw_sin[h];
-  }
-  const bool final_sub = T.upper.nlevels == 0;
-  if (T.nroots == 1) {
-    tier_sub_kernel<NT, true><<<(B + G - 1) / G, 256, smem, s>>>(in, out, T.N, B, T.roots, T.nroots, G, T.sub[0],
-                                                                 T.sub[1], tw, final_sub ? scale : 1.0, swap_in,
-                                                                 final_sub && swap_out);
-  } else {
-    tier_sub_kernel<NT, false><<<T.nroots * B, 256, smem, s>>>(in, out, T.N, B, T.roots, T.nroots, 1, T.sub[0],
-                                                               T.sub[1], tw, final_sub ? scale : 1.0, swap_in,
-                                                               final_sub && swap_out);
-  }
-  for (int lv = 0; lv < T.upper.nlevels; ++lv) {
-    const int n = T.upper.level_n[lv];
-    const long long total = (long long)T.upper.level_count[lv] * (n / 4) * B;
-    const bool last = lv == T.upper.nlevels - 1;
-    tier_level_kernel<NT><<<(int)((total + 255) / 256), 256, 0, s>>>(
-        out, T.N, B, n, T.upper.node_off + T.upper.level_start[lv], T.upper.level_count[lv], tw, last ? scale : 1.0,
-        last && swap_out);
+  const cudaError_t e = nl == 0 ? tier_sub_launch<NT, true>(S, A, s) : tier_sub_launch<NT, false>(S, A, s);
+  if (e != cudaSuccess) return e;
+  const int lgN = 31 - __builtin_clz((unsigned)S.N), step = tier_upper_levels(nl, NT::kLevels);
+  for (int done = 0; done < nl;) {
+    const int r = std::min(step, nl - done), lgu = S.lgT + done - 1, lgnch = lgN - (lgu + r + 1);
+    const bool last = done + r == nl;
+    const unsigned blocks = (unsigned)(((long long)B * (S.N >> (r + 1)) + 255) / 256);
+    const double sc = last ? scale : 1.0;
+    const int sw = last && swap_out;
+    constexpr int R2 = NT::kLevels >= 2 ? 2 : 1, R3 = NT::kLevels >= 3 ? 3 : 1;
+    if (r == 3) tier_upper_kernel<NT, R3><<<blocks, 256, 0, s>>>(A.out, S, B, lgu, lgnch, sc, sw);
+    else if (r == 2) tier_upper_kernel<NT, R2><<<blocks, 256, 0, s>>>(A.out, S, B, lgu, lgnch, sc, sw);
+    else tier_upper_kernel<NT, 1><<<blocks, 256, 0, s>>>(A.out, S, B, lgu, lgnch, sc, sw);
+    done += r;
   }
   return cudaGetLastError();
 }
 
 int tier_words(int tier) { return tier == kTierQD ? 4 : 2; }
 size_t tier_word_bytes(int tier) { return tier == kTierFF ? 4 : 8; }
-int tier_sub_max(int tier) { return tier == kTierQD ? kQDSubMax : tier == kTierFF ? kFFSubMax : kDDSubMax; }
+int tier_sub_max(int tier) {
+  return 1 << (tier == kTierQD ? QDT::kLgMax : tier == kTierFF ? FFT_::kLgMax : DDT::kLgMax);
+}
+int tier_tw_words(int tier) {
+  return tier == kTierQD ? QDT::kTwWords : tier == kTierFF ? FFT_::kTwWords : DDT::kTwWords;
+}
+int tier_leaf_lg(int tier) {
+  return tier == kTierQD ? QDT::kLeafLg : tier == kTierFF ? FFT_::kLeafLg : DDT::kLeafLg;
+}
+int tier_pass_levels(int tier) {
+  return tier == kTierQD ? QDT::kLevels : tier == kTierFF ? FFT_::kLevels : DDT::kLevels;
+}
 
 cudaError_t tier_run_transform(int tier, const DDeviceTables &T, const void *in, void *out, int B, double scale,
                                cudaStream_t s, bool swap_in, bool swap_out) {
@@ -101,11 +146,6 @@ cudaError_t tier_run_transform(int tier, const DDeviceTables &T, const void *in,
     default:
       return cudaErrorInvalidValue;
   }
-}
-
-cudaError_t dd_run_transform(const DDeviceTables &T, const double *in, double *out, int B, double scale,
-                             cudaStream_t s, bool swap_in, bool swap_out) {
-  return tier_run<DDT>(T, in, out, B, scale, s, swap_in, swap_out);
 }
 
 }  // namespace mpfft

@@ -19,20 +19,26 @@
 // rounds it back to a float pair, in FP64 (a float pair is exact in a
 // double), which keeps the products at 2^-52 before the final 2^-48 rounding.
 //
-// Same tree and schedule as the FP64 kernels (d_kernels.cu): maximal nodes of
-// up to T points run in shared memory (DIT-order gather, base cases of at
-// most 4 points, every level up to the node), the levels above in global
-// memory.  T is the largest sub-transform whose planes fit 64 KB: 2048 points
-// for double-double, 1024 for quad-double, 4096 for float-float.  Every level
-// is the 4m2a butterfly with twiddles cos and sin of 2 pi k/N rounded to the
-// tier by MPFR (float-float: to double).  Layout: word (c, h, b, p) at
-// base[((c*K + h)*B + b)*N + p] -- c real/imaginary, h the word, each signal
-// contiguous.
+// Same tree and schedule as the FP64 kernels (d_core.cuh): chunks of up to T
+// output positions run in shared memory, base cases straight from global memory
+// (eight positions a thread: base cases of 4 and 2 points and the 8-point
+// level), then passes that keep a column of points in registers for one level
+// (quad-double), two (double-double) or three (float-float), the last one
+// written out; the levels above run in global memory the same way.  T is the
+// largest chunk whose planes fit 64 KB: 2048 points for double-double, 1024 for
+// quad-double, 4096 for float-float.  Every level is the 4m2a butterfly with
+// twiddles cos and sin of 2 pi k/N rounded to the tier by MPFR (float-float:
+// to double).  Layout: word (c, h, b, p) at base[((c*K + h)*B + b)*N + p] -- c
+// real/imaginary, h the word, each signal contiguous.
+//
+// Every file that includes this is compiled with --fmad=false: an error-free
+// transformation must see the rounded product, not a contracted one.
 #pragma once
 
 #include <cstdint>
 
 #include "mpfft_internal.h"
+#include "sr_chunks.cuh"
 
 namespace mpfft {
 
@@ -84,7 +90,9 @@ struct DDT {
   using V = dd;      // value
   using TW = dd;     // twiddle
   static constexpr int K = 2;
-  static constexpr int kSubMax = kDDSubMax;
+  static constexpr int kLgMax = 11;   // lg of the largest chunk (64 KB)
+  static constexpr int kLeafLg = 3;   // lg of the positions of a base-case slot
+  static constexpr int kLevels = 2;   // levels per pass
 
   // accurate addition (two TwoSums, two renormalisations)
   static __device__ __forceinline__ V add(V x, V y) {
@@ -110,8 +118,23 @@ struct DDT {
     p[0] = v.h;
     p[stride] = v.l;
   }
-  static __device__ __forceinline__ TW twiddle(const double *const *t, size_t k) {
-    return TW{__ldg(t[0] + k), __ldg(t[1] + k)};
+  // shared memory: 16-byte units (re, im) of each word, planes of pl units
+  static constexpr int kUnits = 2;
+  static __device__ __forceinline__ void sload(const double2 *p, int pl, V &r, V &i) {
+    const double2 a = p[0], b = p[pl];
+    r = V{a.x, b.x};
+    i = V{a.y, b.y};
+  }
+  static __device__ __forceinline__ void sstore(double2 *p, int pl, V r, V i) {
+    p[0] = make_double2(r.h, i.h);
+    p[pl] = make_double2(r.l, i.l);
+  }
+  // twiddles: (cos, sin) of each word, planes of len entries
+  static constexpr int kTwWords = 2;
+  static __device__ __forceinline__ void twiddle(const double2 *t, size_t len, TW &c, TW &s) {
+    const double2 a = __ldg(t), b = __ldg(t + len);
+    c = TW{a.x, b.x};
+    s = TW{a.y, b.y};
   }
 };
 
@@ -123,13 +146,11 @@ struct qd {
   double x0, x1, x2, x3;
 };
 
-// Five terms of decreasing order -> four non-overlapping words: a Fast2Sum
+// Four terms of decreasing order -> four non-overlapping words: a Fast2Sum
 // chain from the bottom compresses the terms, a TwoSum chain from the top
 // (exact whatever the magnitudes) pushes what overlaps down again.
-__device__ __forceinline__ qd qd_renorm(double c0, double c1, double c2, double c3, double c4) {
-  dd t = fast_two_sum(c3, c4);
-  c3 = t.h, c4 = t.l;
-  t = fast_two_sum(c2, c3);
+__device__ __forceinline__ qd qd_renorm(double c0, double c1, double c2, double c3) {
+  dd t = fast_two_sum(c2, c3);
   c2 = t.h, c3 = t.l;
   t = fast_two_sum(c1, c2);
   c1 = t.h, c2 = t.l;
@@ -138,8 +159,7 @@ __device__ __forceinline__ qd qd_renorm(double c0, double c1, double c2, double 
   t = two_sum(c1, c2);
   c1 = t.h, c2 = t.l;
   t = two_sum(c2, c3);
-  c2 = t.h, c3 = t.l + c4;
-  return qd{c0, c1, c2, c3};
+  return qd{c0, c1, t.h, t.l};
 }
 
 struct QDT {
@@ -147,7 +167,9 @@ struct QDT {
   using V = qd;
   using TW = qd;
   static constexpr int K = 4;
-  static constexpr int kSubMax = kQDSubMax;
+  static constexpr int kLgMax = 10;
+  static constexpr int kLeafLg = 2;
+  static constexpr int kLevels = 1;
 
   // Sum order by order: word i of x and of y are order i; the error of an
   // order-i TwoSum is order i+1; order 3 is summed plainly (its errors are
@@ -161,7 +183,7 @@ struct QDT {
     const dd u = two_sum(s2.h, s1.l);    // order 2 ...
     const dd t2 = two_sum(u.h, t1.l);
     const double t3 = s3 + s2.l + u.l + t2.l;  // order 3
-    return qd_renorm(s0.h, t1.h, t2.h, t3, 0.0);
+    return qd_renorm(s0.h, t1.h, t2.h, t3);
   }
   static __device__ __forceinline__ V neg(const V &x) { return V{-x.x0, -x.x1, -x.x2, -x.x3}; }
   static __device__ __forceinline__ V sub(const V &x, const V &y) { return add(x, neg(y)); }
@@ -182,7 +204,7 @@ struct QDT {
     const dd y = two_sum(x.h, t.l);
     const dd t2 = two_sum(y.h, t1.l);
     const double t3 = o3 + (p02.l + p11.l + p20.l) + (u.l + v.l + w.l) + (x.l + y.l + t2.l);  // order 3
-    return qd_renorm(p00.h, t1.h, t2.h, t3, 0.0);
+    return qd_renorm(p00.h, t1.h, t2.h, t3);
   }
   static __device__ __forceinline__ V scale(const V &x, double s) { return V{x.x0 * s, x.x1 * s, x.x2 * s, x.x3 * s}; }
   static __device__ __forceinline__ V load(const W *p, size_t stride) {
@@ -194,8 +216,23 @@ struct QDT {
     p[2 * stride] = v.x2;
     p[3 * stride] = v.x3;
   }
-  static __device__ __forceinline__ TW twiddle(const double *const *t, size_t k) {
-    return TW{__ldg(t[0] + k), __ldg(t[1] + k), __ldg(t[2] + k), __ldg(t[3] + k)};
+  static constexpr int kUnits = 4;
+  static __device__ __forceinline__ void sload(const double2 *p, int pl, V &r, V &i) {
+    const double2 a = p[0], b = p[pl], c = p[2 * pl], d = p[3 * pl];
+    r = V{a.x, b.x, c.x, d.x};
+    i = V{a.y, b.y, c.y, d.y};
+  }
+  static __device__ __forceinline__ void sstore(double2 *p, int pl, const V &r, const V &i) {
+    p[0] = make_double2(r.x0, i.x0);
+    p[pl] = make_double2(r.x1, i.x1);
+    p[2 * pl] = make_double2(r.x2, i.x2);
+    p[3 * pl] = make_double2(r.x3, i.x3);
+  }
+  static constexpr int kTwWords = 4;
+  static __device__ __forceinline__ void twiddle(const double2 *t, size_t len, TW &c, TW &s) {
+    const double2 a = __ldg(t), b = __ldg(t + len), e = __ldg(t + 2 * len), d = __ldg(t + 3 * len);
+    c = TW{a.x, b.x, e.x, d.x};
+    s = TW{a.y, b.y, e.y, d.y};
   }
 };
 
@@ -208,7 +245,9 @@ struct FFT_ {
   using V = ff;
   using TW = double;
   static constexpr int K = 2;
-  static constexpr int kSubMax = kFFSubMax;
+  static constexpr int kLgMax = 12;
+  static constexpr int kLeafLg = 3;
+  static constexpr int kLevels = 3;
 
   static __device__ __forceinline__ V add(V a, V b) {
     const ff s = two_sum_f(a.h, b.h);
@@ -228,7 +267,22 @@ struct FFT_ {
     p[0] = v.h;
     p[stride] = v.l;
   }
-  static __device__ __forceinline__ TW twiddle(const double *const *t, size_t k) { return __ldg(t[0] + k); }
+  // one 16-byte unit per point: (re.h, im.h, re.l, im.l)
+  static constexpr int kUnits = 1;
+  static __device__ __forceinline__ void sload(const double2 *p, int, V &r, V &i) {
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    r = V{a.x, a.z};
+    i = V{a.y, a.w};
+  }
+  static __device__ __forceinline__ void sstore(double2 *p, int, V r, V i) {
+    *reinterpret_cast<float4 *>(p) = make_float4(r.h, i.h, r.l, i.l);
+  }
+  static constexpr int kTwWords = 1;
+  static __device__ __forceinline__ void twiddle(const double2 *t, size_t, TW &c, TW &s) {
+    const double2 a = __ldg(t);
+    c = a.x;
+    s = a.y;
+  }
 };
 
 // ---------------------------------------------------------------------------
@@ -275,164 +329,327 @@ __device__ __forceinline__ void bfly(typename NT::V &u0r, typename NT::V &u0i, t
   u0r = a0r, u0i = a0i, u1r = a1r, u1i = a1i, zpr = a2r, zpi = a2i, zmr = a3r, zmi = a3i;
 }
 
-// shared-memory index: low 4 bits XOR-ed with bits 4-7 ^ 8-11, a permutation
-// inside each 16-aligned block (for double-double 17 % fewer wavefronts than
-// padding on this schedule, counted by simulating its accesses)
-__device__ __forceinline__ int swz(int m) { return m ^ (((m >> 4) ^ (m >> 8)) & 15); }
-
-// one shared-memory instance: 2K planes of pl words, [c][h][m]
+// the same with the outputs in the place of the inputs' columns
 template <class NT>
-struct SPlanes {
-  typename NT::W *base;
-  int pl;
-  __device__ typename NT::V re(int m) const { return NT::load(base + swz(m), pl); }
-  __device__ typename NT::V im(int m) const { return NT::load(base + (size_t)NT::K * pl + swz(m), pl); }
-  __device__ void set(int m, typename NT::V r, typename NT::V i) const {
-    NT::store(base + swz(m), pl, r);
-    NT::store(base + (size_t)NT::K * pl + swz(m), pl, i);
-  }
+struct Pt {
+  typename NT::V r, i;
 };
-
-// base cases on positions [o, o+n), in place (n = 4, 2, 1)
 template <class NT>
-__device__ void leaf(const SPlanes<NT> &P, int o, int n) {
-  using V = typename NT::V;
-  if (n == 4) {
-    const V x0r = P.re(o), x1r = P.re(o + 1), x2r = P.re(o + 2), x3r = P.re(o + 3);
-    const V x0i = P.im(o), x1i = P.im(o + 1), x2i = P.im(o + 2), x3i = P.im(o + 3);
-    const V er = NT::add(x0r, x2r), fr = NT::sub(x0r, x2r), gr = NT::add(x1r, x3r), hr = NT::sub(x1r, x3r);
-    const V ei = NT::add(x0i, x2i), fi = NT::sub(x0i, x2i), gi = NT::add(x1i, x3i), hi = NT::sub(x1i, x3i);
-    P.set(o, NT::add(er, gr), NT::add(ei, gi));
-    P.set(o + 1, NT::add(fr, hi), NT::sub(fi, hr));
-    P.set(o + 2, NT::sub(er, gr), NT::sub(ei, gi));
-    P.set(o + 3, NT::sub(fr, hi), NT::add(fi, hr));
-  } else if (n == 2) {
-    const V x0r = P.re(o), x1r = P.re(o + 1), x0i = P.im(o), x1i = P.im(o + 1);
-    P.set(o, NT::add(x0r, x1r), NT::add(x0i, x1i));
-    P.set(o + 1, NT::sub(x0r, x1r), NT::sub(x0i, x1i));
-  }
+__device__ __forceinline__ void bfly(Pt<NT> &u0, Pt<NT> &u1, Pt<NT> &zp, Pt<NT> &zm, typename NT::TW c,
+                                     typename NT::TW s) {
+  bfly<NT>(u0.r, u0.i, u1.r, u1.i, zp.r, zp.i, zm.r, zm.i, c, s);
 }
 
-struct TierTw {
-  const double *c[4], *s[4];  // words of cos and sin of 2 pi k/N, k < N/4
-};
+// DFT of 2 and of 4 points in place (the base cases, reference :108-147)
+template <class NT>
+__device__ __forceinline__ void leaf2(Pt<NT> &a, Pt<NT> &b) {
+  const Pt<NT> x = a, y = b;
+  a = Pt<NT>{NT::add(x.r, y.r), NT::add(x.i, y.i)};
+  b = Pt<NT>{NT::sub(x.r, y.r), NT::sub(x.i, y.i)};
+}
+template <class NT>
+__device__ __forceinline__ void leaf4(Pt<NT> &a, Pt<NT> &b, Pt<NT> &c, Pt<NT> &d) {
+  leaf2<NT>(a, c);  // even samples: a = sum, c = difference
+  leaf2<NT>(b, d);
+  const Pt<NT> e = a, f = c, g = b, h = d;
+  a = Pt<NT>{NT::add(e.r, g.r), NT::add(e.i, g.i)};
+  b = Pt<NT>{NT::add(f.r, h.i), NT::sub(f.i, h.r)};
+  c = Pt<NT>{NT::sub(e.r, g.r), NT::sub(e.i, g.i)};
+  d = Pt<NT>{NT::sub(f.r, h.i), NT::add(f.i, h.r)};
+}
 
-// One CTA = G instances (sub-transform root x signal) in shared memory; see
-// d_sub_kernel (d_kernels.cu) for the schedule.  swap_in / swap_out: read the
-// input's / write the output's real and imaginary planes exchanged.
-template <class NT, bool SINGLE>
-__device__ __forceinline__ void tier_sub_instances(const typename NT::W *__restrict__ in,
-                                                   typename NT::W *__restrict__ out, int N, int B, int b0, int G_here,
-                                                   SubRoot rt, const SubSchedule &big, const SubSchedule &small,
-                                                   const TierTw &tw, double scale, int swap_in, int swap_out,
-                                                   typename NT::W *sm) {
-  using W = typename NT::W;
-  using V = typename NT::V;
-  constexpr int K = NT::K;
-  const int Tmax = big.size;
-  const int lgT = 31 - __clz(Tmax);
-  const int pl = Tmax;  // plane length
-  const int tws = N / Tmax;
-  const bool is_big = SINGLE || rt.size == Tmax;
-  const int T = rt.size;
-  const int *perm = is_big ? big.perm : small.perm;
-  const Leaf *leaves = is_big ? big.leaves : small.leaves;
-  const int nleaves = is_big ? big.nleaves : small.nleaves;
-  const int nlevels = is_big ? big.nlevels : small.nlevels;
-  auto inst = [&](int g) { return SPlanes<NT>{sm + (size_t)g * 2 * K * pl, pl}; };
-  const size_t hplane = (size_t)B * N;          // word h -> word h+1
-  const size_t cplane = (size_t)K * hplane;     // real -> imaginary component
-  const size_t in_re = swap_in ? cplane : 0, in_im = swap_in ? 0 : cplane;
-  const size_t out_re = swap_out ? cplane : 0, out_im = swap_out ? 0 : cplane;
-  // gather: element j of instance g to DIT position perm[j], 4 elements per thread in flight
-  const int total = G_here << lgT;
-  for (int e0 = 0; e0 < total; e0 += 4 * (int)blockDim.x) {
-    V vr[4], vi[4];
-    int dst[4], gg[4];
+// the butterfly of an 8-point node at k = 0 (twiddle 1)
+template <class NT>
+__device__ __forceinline__ void leaf8_k0(Pt<NT> &u0, Pt<NT> &u1, Pt<NT> &zp, Pt<NT> &zm) {
+  const Pt<NT> a = u0, b = u1;
+  const typename NT::V sr = NT::add(zp.r, zm.r), si = NT::add(zp.i, zm.i);
+  const typename NT::V dr = NT::sub(zp.r, zm.r), di = NT::sub(zp.i, zm.i);
+  u0 = Pt<NT>{NT::add(a.r, sr), NT::add(a.i, si)};
+  zp = Pt<NT>{NT::sub(a.r, sr), NT::sub(a.i, si)};
+  u1 = Pt<NT>{NT::add(b.r, di), NT::sub(b.i, dr)};
+  zm = Pt<NT>{NT::sub(b.r, di), NT::add(b.i, dr)};
+}
+
+// twiddle k of node size n: entry tier_level_tw(n) + k of the table of all levels n = 8 .. N
+__host__ __device__ inline int tier_level_tw(int n) { return n / 4 - 2; }
+
+template <class NT>
+__device__ __forceinline__ void tier_tw(const TierTab &S, int n, int k, typename NT::TW &c, typename NT::TW &s) {
+  NT::twiddle(S.tw + tier_level_tw(n) + k, S.tw_len, c, s);
+}
+
+// R levels of one column in registers: d_levels (d_core.cuh) for a tier
+template <class NT, int R>
+__device__ __forceinline__ void tier_levels(Pt<NT> (&v)[2 << R], bool big, const TierTab &S, int u, int k) {
+  typename NT::TW c, s;
+  if constexpr (R == 1) {
+    if (!big) return;
+    tier_tw<NT>(S, 4 * u, k, c, s);
+    bfly<NT>(v[0], v[1], v[2], v[3], c, s);
+  } else if constexpr (R == 2) {
+    tier_tw<NT>(S, 4 * u, k, c, s);
+    bfly<NT>(v[0], v[1], v[2], v[3], c, s);
+    if (big) {
+      tier_tw<NT>(S, 8 * u, k, c, s);
+      bfly<NT>(v[0], v[2], v[4], v[6], c, s);
+      tier_tw<NT>(S, 8 * u, k + u, c, s);
+      bfly<NT>(v[1], v[3], v[5], v[7], c, s);
+    } else {
+      bfly<NT>(v[4], v[5], v[6], v[7], c, s);
+    }
+  } else {
+    tier_tw<NT>(S, 4 * u, k, c, s);
+    bfly<NT>(v[0], v[1], v[2], v[3], c, s);
+    bfly<NT>(v[8], v[9], v[10], v[11], c, s);
+    if (big) bfly<NT>(v[12], v[13], v[14], v[15], c, s);
+    tier_tw<NT>(S, 8 * u, k, c, s);
+    bfly<NT>(v[0], v[2], v[4], v[6], c, s);
+    if (!big) bfly<NT>(v[8], v[10], v[12], v[14], c, s);
+    tier_tw<NT>(S, 8 * u, k + u, c, s);
+    bfly<NT>(v[1], v[3], v[5], v[7], c, s);
+    if (!big) bfly<NT>(v[9], v[11], v[13], v[15], c, s);
+    if (big) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = e0 + u * (int)blockDim.x + (int)threadIdx.x;
-      const int g = e >> lgT, j = e & (Tmax - 1);
-      dst[u] = -1;
-      gg[u] = g;
-      if (e < total && (SINGLE || j < T)) {
-        int idx = rt.sn + j * rt.s;
-        if (idx < 0) idx += N;
-        const size_t o = (size_t)(b0 + g) * N + idx;
-        vr[u] = NT::load(in + in_re + o, hplane);
-        vi[u] = NT::load(in + in_im + o, hplane);
-        dst[u] = perm[j];
+      for (int i = 0; i < 4; ++i) {
+        tier_tw<NT>(S, 16 * u, k + i * u, c, s);
+        bfly<NT>(v[i], v[i + 4], v[i + 8], v[i + 12], c, s);
       }
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (dst[u] >= 0) inst(gg[u]).set(dst[u], vr[u], vi[u]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < G_here * nleaves; e += blockDim.x) {
-    const int g = SINGLE ? e / nleaves : 0, l = SINGLE ? e - g * nleaves : e;
-    const Leaf lf = leaves[l];
-    leaf<NT>(inst(g), lf.out, lf.n);
-  }
-  for (int lv = 0; lv < nlevels; ++lv) {
-    __syncthreads();
-    const int n = big.level_n[lv], q = n >> 2, lgq = 29 - __clz(n);
-    const int cnt = is_big ? big.level_count[lv] : small.level_count[lv];
-    const int *nodes = (is_big ? big.node_off : small.node_off) + (is_big ? big.level_start[lv] : small.level_start[lv]);
-    const int per = cnt * q;
-    for (int e = threadIdx.x; e < G_here * per; e += blockDim.x) {
-      const int g = SINGLE ? e / per : 0, t = SINGLE ? e - g * per : e;
-      const int node = t >> lgq, k = t & (q - 1);
-      const size_t km = (size_t)(k << (lgT - (lgq + 2))) * tws;  // k * (N/n)
-      const SPlanes<NT> P = inst(g);
-      const int off = nodes[node];
-      V u0r = P.re(off + k), u0i = P.im(off + k), u1r = P.re(off + k + q), u1i = P.im(off + k + q);
-      V zpr = P.re(off + k + 2 * q), zpi = P.im(off + k + 2 * q), zmr = P.re(off + k + 3 * q),
-        zmi = P.im(off + k + 3 * q);
-      bfly<NT>(u0r, u0i, u1r, u1i, zpr, zpi, zmr, zmi, NT::twiddle(tw.c, km), NT::twiddle(tw.s, km));
-      P.set(off + k, u0r, u0i);
-      P.set(off + k + q, u1r, u1i);
-      P.set(off + k + 2 * q, zpr, zpi);
-      P.set(off + k + 3 * q, zmr, zmi);
-    }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int g = e >> lgT, m = e & (Tmax - 1);
-    if (!SINGLE && m >= T) continue;
-    const SPlanes<NT> P = inst(g);
-    const size_t o = (size_t)(b0 + g) * N + rt.out + m;
-    NT::store(out + out_re + o, hplane, NT::scale(P.re(m), scale));
-    NT::store(out + out_im + o, hplane, NT::scale(P.im(m), scale));
   }
 }
 
-// butterfly k of the node at offset off (size n) of signal b, above the
-// shared-memory sub-transforms (in place in global memory)
+// shared-memory index of the 16-byte units (as d_swz in d_core.cuh)
+__device__ __forceinline__ int tier_swz(int m) { return m ^ (((m >> 3) ^ (m >> 6) ^ (m >> 9)) & 7); }
+
+// One CTA's sub-transforms, as in d_core.cuh: SINGLE: G whole signals b0 ..;
+// otherwise G chunks (input classes c0 ..) of signal b0.
 template <class NT>
-__device__ __forceinline__ void tier_level_one(typename NT::W *__restrict__ y, int N, int B, int n, int off, int k,
-                                               int b, const TierTw &tw, double scale, int swap_out) {
-  using W = typename NT::W;
-  using V = typename NT::V;
-  const int q = n >> 2;
-  off += k;
-  const size_t hplane = (size_t)B * N, cplane = (size_t)NT::K * hplane;
-  W *re = y + (size_t)b * N, *im = y + cplane + (size_t)b * N;
-  V u0r = NT::load(re + off, hplane), u0i = NT::load(im + off, hplane);
-  V u1r = NT::load(re + off + q, hplane), u1i = NT::load(im + off + q, hplane);
-  V zpr = NT::load(re + off + 2 * q, hplane), zpi = NT::load(im + off + 2 * q, hplane);
-  V zmr = NT::load(re + off + 3 * q, hplane), zmi = NT::load(im + off + 3 * q, hplane);
-  const size_t km = (size_t)k * (N / n);
-  bfly<NT>(u0r, u0i, u1r, u1i, zpr, zpi, zmr, zmi, NT::twiddle(tw.c, km), NT::twiddle(tw.s, km));
-  W *ore = swap_out ? im : re, *oim = swap_out ? re : im;
-  NT::store(ore + off, hplane, NT::scale(u0r, scale));
-  NT::store(oim + off, hplane, NT::scale(u0i, scale));
-  NT::store(ore + off + q, hplane, NT::scale(u1r, scale));
-  NT::store(oim + off + q, hplane, NT::scale(u1i, scale));
-  NT::store(ore + off + 2 * q, hplane, NT::scale(zpr, scale));
-  NT::store(oim + off + 2 * q, hplane, NT::scale(zpi, scale));
-  NT::store(ore + off + 3 * q, hplane, NT::scale(zmr, scale));
-  NT::store(oim + off + 3 * q, hplane, NT::scale(zmi, scale));
+struct TierArgs {
+  const typename NT::W *in;
+  typename NT::W *out;
+  int B, b0, c0, G;
+  int per;  // levels per pass, up to kLevels
+  double scale;
+  bool final, swap_in, swap_out;
+};
+
+// What it takes (a gather pass, base cases of 4 points and one
+// level per pass, one level per launch above / this; us): double-double 4096
+// points x 512 171 / 139, 65536 x 32 266 / 197 -- half of the FP64 pipe's rate at
+// 376 operations a butterfly; quad-double 4096 x 512 640 / 564; float-float 4096 x
+// 512 84 / 52, 2^20 x 2 210 / 115 (memory).
+//
+// Base cases from global memory, one thread per slot of 2^kLeafLg output
+// positions; either way the slot's inputs are of one class mod N/2^kLeafLg:
+//   8  a node of 8 points (a leaf of 4, two of 2, and the level above) or two leaves of 4
+//   4  a leaf of 4 or two of 2 (quad-double: eight points do not fit in registers)
+template <class NT, bool SINGLE>
+__device__ __forceinline__ void tier_leaves(const TierTab &S, const TierArgs<NT> &A, double2 *sm) {
+  constexpr int kLg = NT::kLeafLg, kPts = 1 << kLg;
+  const int lgT = S.lgT, nslots = 1 << (lgT - kLg), pl = A.G << lgT, N = S.N;
+  const size_t hplane = (size_t)A.B * N, cplane = (size_t)NT::K * hplane;
+  const size_t in_re = A.swap_in ? cplane : 0, in_im = A.swap_in ? 0 : cplane;
+  for (int e = threadIdx.x; e < A.G * nslots; e += blockDim.x) {
+    const int g = SINGLE ? e / nslots : e % A.G;
+    int s = SINGLE ? e % nslots : e / A.G;
+    int half = 0, sna = 0, rs = 1, chunk = 0;
+    const TierLeafSlot *tab = S.slots[0];
+    if (!SINGLE) {
+      const SrChunk ch = S.chunks[A.c0 + g];
+      chunk = ch.chunk;
+      sna = ch.sna;
+      rs = N >> lgT;
+      if (!sr_chunk_big(chunk)) {
+        tab = S.slots[1];
+        rs *= 2;
+        half = s >= nslots / 2;
+        s -= half ? nslots / 2 : 0;
+        if (half) sna = ch.snb;
+      }
+    }
+    const TierLeafSlot L = tab[s];
+    const int m = half * (nslots / 2) + L.m;
+    const bool big = sr_chunk_big(chunk * nslots + m);
+    const int a0 = sna + L.in[0] * rs, a1 = sna + L.in[1] * rs, a2 = sna + L.in[2] * rs, st = N >> 2;
+    const size_t sig = (size_t)(SINGLE ? A.b0 + g : A.b0) * N;
+    Pt<NT> v[kPts];
+#pragma unroll
+    for (int j = 0; j < kPts; ++j) {
+      int idx;
+      if (kPts == 8)  // block 0: a leaf of 4; block 1: a leaf of 4, or two of 2 points with stride N/2
+        idx = j < 4 ? a0 + j * st : !big ? a1 + (j - 4) * st : (j < 6 ? a1 : a2) + 2 * (j & 1) * st;
+      else
+        idx = big ? a0 + j * st : (j < 2 ? a0 : a1) + 2 * (j & 1) * st;
+      if (idx < 0) idx += N;
+      v[j].r = NT::load(A.in + in_re + sig + idx, hplane);
+      v[j].i = NT::load(A.in + in_im + sig + idx, hplane);
+    }
+    if constexpr (kPts == 8) {
+      leaf4<NT>(v[0], v[1], v[2], v[3]);
+      if (big) {
+        leaf2<NT>(v[4], v[5]);
+        leaf2<NT>(v[6], v[7]);
+        // level of 8 points: k = 0 has no products, k = 1 the twiddle of 1/8 turn
+        leaf8_k0<NT>(v[0], v[2], v[4], v[6]);
+        typename NT::TW c, sn;
+        tier_tw<NT>(S, 8, 1, c, sn);
+        bfly<NT>(v[1], v[3], v[5], v[7], c, sn);
+      } else {
+        leaf4<NT>(v[4], v[5], v[6], v[7]);
+      }
+    } else if (big) {
+      leaf4<NT>(v[0], v[1], v[2], v[3]);
+    } else {
+      leaf2<NT>(v[0], v[1]);
+      leaf2<NT>(v[2], v[3]);
+    }
+    const int at = tier_swz((g << lgT) + kPts * m);
+#pragma unroll
+    for (int j = 0; j < kPts; ++j) NT::sstore(sm + (at ^ tier_swz(j)), pl, v[j].r, v[j].i);
+  }
+}
+
+// a point of the transform's output (or of the levels below the upper ones)
+template <class NT>
+__device__ __forceinline__ void tier_put(typename NT::W *re, typename NT::W *im, size_t hplane, const Pt<NT> &v,
+                                         double scale) {
+  NT::store(re, hplane, NT::scale(v.r, scale));
+  NT::store(im, hplane, NT::scale(v.i, scale));
+}
+
+// The chunks of a granularity by type, so that a warp's lanes mostly take the
+// same branch: chunk indexes that are one node, ascending, at order[0 ..], those
+// that are pairs at order[kOrderPairs ..] (by the index inside the sub-transform:
+// in one that is itself a pair, its last chunk has the other type).
+constexpr int kOrder = 272, kOrderPairs = 176;  // up to 256 chunks (16 of 4096 points), 171 nodes and 85 pairs
+constexpr size_t kOrderBytes = kOrder * sizeof(uint16_t);
+
+__device__ __forceinline__ uint16_t *tier_order(double2 *sm, int units) { return reinterpret_cast<uint16_t *>(sm + units); }
+
+__device__ __forceinline__ void tier_fill_order(uint16_t *order, int chunks) {
+  for (int m = threadIdx.x; m < chunks; m += blockDim.x) {
+    int rank = 0;  // nodes below m
+    for (int s = 0; m >> s; ++s) rank += (s & 1) ? -(m >> s) : (m >> s);
+    if (sr_chunk_big(m)) order[rank] = (uint16_t)m;
+    else order[kOrderPairs + m - rank] = (uint16_t)m;
+  }
+}
+
+// R levels of every chunk of 2^(R+1)*u positions, u = 2^lgu; last: to global memory
+template <class NT, int R, bool SINGLE>
+__device__ __forceinline__ void tier_pass(const TierTab &S, const TierArgs<NT> &A, double2 *sm, int lgu, bool last) {
+  constexpr int M = 2 << R;
+  const int lgT = S.lgT, pl = A.G << lgT, u = 1 << lgu, lgc = lgu + R + 1, lgnch = lgT - lgc;
+  const size_t hplane = (size_t)A.B * S.N, cplane = (size_t)NT::K * hplane;
+  int off[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) off[j] = tier_swz(j << lgu);
+  const uint16_t *order = tier_order(sm, pl * NT::kUnits);
+  const int nch = 1 << lgnch, nodes = ((2 << lgnch) + ((lgnch & 1) ? -1 : 1)) / 3;
+  // one level alone only has work in the nodes (and in a pair's last chunk, see above)
+  const bool only = R == 1 && !last;
+  const int slots = only ? nodes + (!SINGLE && (lgnch & 1) ? 1 : 0) : nch;
+  for (int e = threadIdx.x; e < (A.G * slots) << lgu; e += blockDim.x) {
+    const int k = e & (u - 1), x = e >> lgu, g = only ? x / slots : x >> lgnch, i = x - g * slots;
+    const int ci = i < nodes ? order[i] : only ? nch - 1 : order[kOrderPairs + i - nodes], c = (g << lgnch) + ci;
+    const int chunk = SINGLE ? 0 : __ldg(&S.chunks[A.c0 + g].chunk);
+    const bool big = sr_chunk_big((chunk << lgnch) + ci);
+    if (only && !big) continue;
+    const int at = tier_swz((c << lgc) + k);
+    Pt<NT> v[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) NT::sload(sm + (at ^ off[j]), pl, v[j].r, v[j].i);
+    tier_levels<NT, R>(v, big, S, u, k);
+    if (!last) {
+#pragma unroll
+      for (int j = 0; j < M; ++j) NT::sstore(sm + (at ^ off[j]), pl, v[j].r, v[j].i);
+    } else {
+      const size_t p = (size_t)(SINGLE ? A.b0 + g : A.b0) * S.N + ((size_t)chunk << lgT) + ((size_t)ci << lgc) + k;
+      typename NT::W *re = A.out + (A.swap_out ? cplane : 0) + p, *im = A.out + (A.swap_out ? 0 : cplane) + p;
+      const double sc = A.final ? A.scale : 1.0;
+#pragma unroll
+      for (int j = 0; j < M; ++j) tier_put<NT>(re + ((size_t)j << lgu), im + ((size_t)j << lgu), hplane, v[j], sc);
+    }
+  }
+}
+
+// T = 2^lgT >= 8
+template <class NT, bool SINGLE>
+__device__ __forceinline__ void tier_sub_transform(const TierTab &S, const TierArgs<NT> &A, double2 *sm) {
+  tier_fill_order(tier_order(sm, (A.G << S.lgT) * NT::kUnits), 1 << (S.lgT - NT::kLeafLg) >> 1);
+  tier_leaves<NT, SINGLE>(S, A, sm);
+  int done = NT::kLeafLg;
+  if (done == S.lgT) {  // (8 points) the base cases are the transform
+    __syncthreads();
+    const size_t hplane = (size_t)A.B * S.N, cplane = (size_t)NT::K * hplane;
+    for (int e = threadIdx.x; e < A.G * 8; e += blockDim.x) {
+      Pt<NT> v;
+      NT::sload(sm + tier_swz(e), A.G * 8, v.r, v.i);
+      typename NT::W *o = A.out + (size_t)A.b0 * 8 + e;
+      tier_put<NT>(o + (A.swap_out ? cplane : 0), o + (A.swap_out ? 0 : cplane), hplane, v, A.final ? A.scale : 1.0);
+    }
+    return;
+  }
+  while (done < S.lgT) {
+    const int r = min(A.per, S.lgT - done);
+    const bool last = done + r == S.lgT;
+    __syncthreads();
+    if (NT::kLevels == 3 && r == 3) tier_pass<NT, NT::kLevels, SINGLE>(S, A, sm, done - 1, last);
+    else if (NT::kLevels >= 2 && r == 2) tier_pass<NT, NT::kLevels >= 2 ? 2 : 1, SINGLE>(S, A, sm, done - 1, last);
+    else tier_pass<NT, 1, SINGLE>(S, A, sm, done - 1, last);
+    done += r;
+  }
+}
+
+// transforms of N <= 4 points: signal b0 + g
+template <class NT>
+__device__ __forceinline__ void tier_tiny(const TierTab &S, const TierArgs<NT> &A) {
+  const size_t hplane = (size_t)A.B * S.N, cplane = (size_t)NT::K * hplane;
+  for (int g = threadIdx.x; g < A.G; g += blockDim.x) {
+    const size_t sig = (size_t)(A.b0 + g) * S.N;
+    const typename NT::W *re = A.in + (A.swap_in ? cplane : 0) + sig, *im = A.in + (A.swap_in ? 0 : cplane) + sig;
+    typename NT::W *ore = A.out + (A.swap_out ? cplane : 0) + sig, *oim = A.out + (A.swap_out ? 0 : cplane) + sig;
+    Pt<NT> v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int p = min(j, S.N - 1);
+      v[j] = Pt<NT>{NT::load(re + p, hplane), NT::load(im + p, hplane)};
+    }
+    if (S.N == 4) leaf4<NT>(v[0], v[1], v[2], v[3]);
+    else if (S.N == 2) leaf2<NT>(v[0], v[1]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (j < S.N) tier_put<NT>(ore + j, oim + j, hplane, v[j], A.scale);
+  }
+}
+
+// R levels above the sub-transforms: column k of chunk c of signal b, in place
+// in global memory
+template <class NT, int R>
+__device__ __forceinline__ void tier_upper_column(typename NT::W *__restrict__ y, const TierTab &S, int B, int lgu, int b,
+                                                  int c, int k, double scale, bool swap_out) {
+  constexpr int M = 2 << R;
+  const size_t hplane = (size_t)B * S.N, cplane = (size_t)NT::K * hplane;
+  const bool big = sr_chunk_big(c);
+  if (R == 1 && !big) return;  // (never the last level: its chunk is the root)
+  typename NT::W *re = y + (size_t)b * S.N + ((size_t)c << (lgu + R + 1)) + k, *im = re + cplane;
+  Pt<NT> v[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) {
+    v[j].r = NT::load(re + ((size_t)j << lgu), hplane);
+    v[j].i = NT::load(im + ((size_t)j << lgu), hplane);
+  }
+  tier_levels<NT, R>(v, big, S, 1 << lgu, k);
+  typename NT::W *ore = swap_out ? im : re, *oim = swap_out ? re : im;
+#pragma unroll
+  for (int j = 0; j < M; ++j) tier_put<NT>(ore + ((size_t)j << lgu), oim + ((size_t)j << lgu), hplane, v[j], scale);
+}
+
+// levels above the sub-transforms per pass: the fewest passes of at most
+// `most` levels, evenly
+__host__ __device__ inline int tier_upper_levels(int nl, int most) {
+  const int passes = (nl + most - 1) / most;
+  return passes ? (nl + passes - 1) / passes : 0;
 }
 
 }  // namespace mpfft

@@ -416,11 +416,10 @@ static int mp_limbs_for(unsigned long N, long P) {
 
 struct MpTwiddles {
   uint32_t *d_tw = nullptr;
-  uint32_t *d_twp = nullptr;  // packed copy (mp_pack_tw), up to kMaxLimbs limbs
+  uint32_t *d_twp = nullptr;  // packed copy (mp_pack_tw) behind the table, up to kMaxLimbs limbs
   uint8_t *d_dneg = nullptr;
   ~MpTwiddles() {
     if (d_tw) cudaFree(d_tw);
-    if (d_twp) cudaFree(d_twp);
     if (d_dneg) cudaFree(d_dneg);
   }
 };
@@ -462,8 +461,14 @@ static int build_twiddles(MpTwiddles &tw, unsigned long N, int L) {
     mpfr_clear(t);
     mpfr_free_cache();
   });
-  CUDA_TRY(cudaMalloc(&tw.d_tw, h.size() * sizeof(uint32_t)));
+  const bool pack = L <= kMaxLimbs;
+  const size_t at = (h.size() + 3) & ~(size_t)3;  // (the packed copy is read in 16-byte units)
+  CUDA_TRY(cudaMalloc(&tw.d_tw, (at + (pack ? mp_packed_tw_words(L, (long long)q) : 0)) * sizeof(uint32_t)));
   CUDA_TRY(cudaMemcpy(tw.d_tw, h.data(), h.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  if (pack) {
+    tw.d_twp = tw.d_tw + at;
+    CUDA_TRY(mp_pack_tw(tw.d_tw, tw.d_twp, L, (long long)q, nullptr));  // done before the next copy returns
+  }
   CUDA_TRY(cudaMalloc(&tw.d_dneg, q));
   CUDA_TRY(cudaMemcpy(tw.d_dneg, neg.data(), q, cudaMemcpyHostToDevice));
   return MPFFT_OK;
@@ -595,7 +600,6 @@ struct mpfft_d_plan {
   bool real = false;        // real transform of n_real = 2N points: N-point complex transform + split step
   unsigned long n_real = 0;
   double *d_wc = nullptr, *d_ws = nullptr;  // real plans: cos, sin of 2 pi k / n_real, k < N/2
-  DeviceTree upper;                   // levels above the shared-memory sub-transforms
   std::vector<void *> dev_allocs;     // roots, perms, sub-schedule tables
   DDeviceTables tabs;
   cudaStream_t stream = nullptr;
@@ -679,14 +683,9 @@ static int mp_plan_init(mpfft_mp_plan *p, unsigned long n, long prec, bool host_
   static_cast<TreeTables &>(p->tabs) = p->tree.tabs;
   p->tabs.tw = p->tw.d_tw;
   p->tabs.dneg = p->tw.d_dneg;
+  p->tabs.twp = p->tw.d_twp;
   p->tabs.tws = real ? 2 : 1;
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
-  if (L <= kMaxLimbs && nt >= 16) {
-    CUDA_TRY(cudaMalloc(&p->tw.d_twp, mp_packed_tw_words(L, (long long)n / 4) * sizeof(uint32_t)));
-    CUDA_TRY(mp_pack_tw(p->tw.d_tw, p->tw.d_twp, L, (long long)n / 4, p->stream));
-    CUDA_TRY(cudaStreamSynchronize(p->stream));
-    p->tabs.twp = p->tw.d_twp;
-  }
   return MPFFT_OK;
 }
 
@@ -1353,79 +1352,26 @@ static int upload(mpfft_d_plan *p, const std::vector<T> &v, const T **out) {
   return MPFFT_OK;
 }
 
-// Schedule of a shared-memory sub-transform of `size` points: the leaves and
-// levels of its own recursion tree, and the DIT input order perm[m].
-static int build_sub(mpfft_d_plan *p, int size, SubSchedule &S, int leaf_max = 16) {
-  HostTree t;
-  walk(t, size, 1, 0, 0, leaf_max);
-  // invperm[j] = DIT position of element j of the sub-transform's input sequence
-  std::vector<int> perm(size);
-  for (const Leaf &lf : t.leaves)
-    for (int j = 0; j < lf.n; ++j) perm[(j == 0 && lf.sn < 0) ? lf.sn + size : lf.sn + j * lf.s] = lf.out + j;
-  std::vector<int> nodes;
-  std::stable_sort(t.leaves.begin(), t.leaves.end(), [](const Leaf &a, const Leaf &b) { return a.n > b.n; });
-  S.size = size;
-  S.nleaves = (int)t.leaves.size();
-  S.nleaf16 = (int)std::count_if(t.leaves.begin(), t.leaves.end(), [](const Leaf &l) { return l.n == 16; });
-  S.nleaf8 = (int)std::count_if(t.leaves.begin(), t.leaves.end(), [](const Leaf &l) { return l.n == 8; });
-  S.nlevels = 0;
-  for (auto &kv : t.levels) {
-    if (S.nlevels >= kMaxLevels) return set_err(MPFFT_EUNSUPPORTED, "sub-transform too large");
-    S.level_n[S.nlevels] = kv.first;
-    S.level_start[S.nlevels] = (int)nodes.size();
-    S.level_count[S.nlevels] = (int)kv.second.size();
-    nodes.insert(nodes.end(), kv.second.begin(), kv.second.end());
-    ++S.nlevels;
-  }
-  // per level: its nodes that are not the first child of a node of the next
-  // level (a first child starts at its parent's offset)
-  std::vector<int> pair_nodes;
-  for (int l = 0; l + 1 < S.nlevels; ++l) {
-    const int *up = nodes.data() + S.level_start[l + 1];
-    std::set<int> parents(up, up + S.level_count[l + 1]);
-    S.pair_start[l] = (int)pair_nodes.size();
-    for (int j = 0; j < S.level_count[l]; ++j) {
-      const int o = nodes[S.level_start[l] + j];
-      if (!parents.count(o)) pair_nodes.push_back(o);
-    }
-    S.pair_count[l] = (int)pair_nodes.size() - S.pair_start[l];
-  }
-  if (int e = upload(p, perm, &S.perm)) return e;
-  if (int e = upload(p, t.leaves, &S.leaves)) return e;
-  if (int e = upload(p, nodes, &S.node_off)) return e;
-  if (int e = upload(p, pair_nodes, &S.pair_nodes)) return e;
-  return MPFFT_OK;
-}
-
-// Base cases of a T-point tree (T >= 32), one slot per 16 output positions,
-// ordered so that a warp's loads are of neighbouring input classes (16-point
-// leaves first) and its eight-lane shared-memory phases hit different banks
-// where the window of 32 slots allows it (key: the swizzled position's low 3
-// bits, d_swz in d_core.cuh).
-static std::vector<SrLeafSlot> leaf_slots(int T) {
-  HostTree t;
-  walk(t, T, 1, 0, 0, 16);
-  std::vector<SrLeafSlot> slots(T / 16);
-  for (const Leaf &lf : t.leaves) {
-    SrLeafSlot &s = slots[lf.out / 16];
-    s.m = lf.out / 16;
-    if (lf.out % 16 == 0) s.sna = lf.sn;
-    else s.snb = lf.sn;
-  }
-  auto cls = [&](const SrLeafSlot &s) { return ((s.sna % (T / 16)) + T / 16) % (T / 16); };
-  std::stable_sort(slots.begin(), slots.end(), [&](const SrLeafSlot &a, const SrLeafSlot &b) {
+// Orders the base-case slots of a T-point tree (blk output positions each) so
+// that a warp's loads are of neighbouring input classes (blocks that are one
+// node first) and its eight-lane shared-memory phases hit different banks where
+// the window of 32 slots allows it (key: the swizzled position's low 3 bits,
+// d_swz in d_core.cuh).  class_of: input class of a slot mod T/blk.
+template <class Slot, class F>
+static std::vector<Slot> order_slots(std::vector<Slot> slots, int blk, F class_of) {
+  std::stable_sort(slots.begin(), slots.end(), [&](const Slot &a, const Slot &b) {
     const bool ba = sr_chunk_big(a.m), bb = sr_chunk_big(b.m);
-    return ba != bb ? ba : cls(a) < cls(b);
+    return ba != bb ? ba : class_of(a) < class_of(b);
   });
-  std::vector<SrLeafSlot> out;
+  std::vector<Slot> out;
   for (size_t w = 0; w < slots.size(); w += 32) {
     const size_t e = std::min(slots.size(), w + 32);
     for (int big = 1; big >= 0; --big) {
-      std::vector<SrLeafSlot> bank[8];
+      std::vector<Slot> bank[8];
       size_t left = 0;
       for (size_t i = w; i < e; ++i)
         if (sr_chunk_big(slots[i].m) == (big != 0)) {
-          const int m = 16 * slots[i].m;
+          const int m = blk * slots[i].m;
           bank[((m >> 3) ^ (m >> 6) ^ (m >> 9)) & 7].push_back(slots[i]);
           ++left;
         }
@@ -1444,36 +1390,84 @@ static std::vector<SrLeafSlot> leaf_slots(int T) {
   return out;
 }
 
-// lg of the sub-transform size of an N-point FP64 transform longer than
-// kDSubMax: the smallest of 1024, 2048 and 4096 points that needs no more
-// passes of three levels above it than the others (smaller chunks let a CTA
-// hold several of neighbouring input classes).
-static int d_sub_lg(int lgN) {
-  int best = 12;
-  for (int l = 11; l >= 10; --l)
-    if ((lgN - l + 2) / 3 <= (lgN - best + 2) / 3) best = l;
+// FP64 base cases of a T-point tree (T >= 32), one slot per 16 output positions
+static std::vector<SrLeafSlot> leaf_slots(int T) {
+  HostTree t;
+  walk(t, T, 1, 0, 0, 16);
+  std::vector<SrLeafSlot> slots(T / 16);
+  for (const Leaf &lf : t.leaves) {
+    SrLeafSlot &s = slots[lf.out / 16];
+    s.m = lf.out / 16;
+    if (lf.out % 16 == 0) s.sna = lf.sn;
+    else s.snb = lf.sn;
+  }
+  const int cls = T / 16;
+  return order_slots(slots, 16, [cls](const SrLeafSlot &s) { return ((s.sna % cls) + cls) % cls; });
+}
+
+// base cases of a tier's T-point tree (T >= 8), one slot per blk = 8 or 4 output positions
+static std::vector<TierLeafSlot> tier_leaf_slots(int T, int blk) {
+  HostTree t;
+  walk(t, T, 1, 0, 0, 4);
+  std::vector<TierLeafSlot> slots(T / blk);
+  for (const Leaf &lf : t.leaves) {
+    TierLeafSlot &s = slots[lf.out / blk];
+    const int at = lf.out % blk;
+    s.m = lf.out / blk;
+    s.in[blk == 8 ? (at == 0 ? 0 : at == 4 ? 1 : 2) : at / 2] = lf.sn;
+  }
+  const int cls = T / blk;
+  return order_slots(slots, blk, [cls](const TierLeafSlot &s) { return ((s.in[0] % cls) + cls) % cls; });
+}
+
+// chunks of T output positions of an n-point tree by input class mod n/T
+static std::vector<SrChunk> tree_chunks(int n, int T) {
+  HostTree t;
+  walk(t, n, 1, 0, 0, T);
+  const int nc = n / T;
+  std::vector<SrChunk> chunks(nc);
+  for (const Leaf &lf : t.leaves) {
+    SrChunk &c = chunks[lf.out / T];
+    c.chunk = lf.out / T;
+    if (lf.out % T == 0) c.sna = lf.sn;
+    else c.snb = lf.sn;
+  }
+  auto cls = [nc](const SrChunk &c) { return ((c.sna % nc) + nc) % nc; };
+  std::stable_sort(chunks.begin(), chunks.end(), [&](const SrChunk &a, const SrChunk &b) { return cls(a) < cls(b); });
+  return chunks;
+}
+
+// lg of the sub-transform size T of a 2^lgN-point transform: all of it up to
+// `most`, else the smallest of lo .. most that needs no more passes of `per`
+// levels above it than the others (smaller chunks let a CTA hold several of
+// neighbouring input classes).  A given sub_max > 0 instead rounds down to one of
+// lo .. most.
+static int sub_lg(int lgN, int lo, int most, int per, int sub_max) {
+  if (lgN <= lo) return lgN;
+  if (sub_max > 0) {
+    int l = lo;
+    while (l < most && (2 << l) <= sub_max) ++l;
+    return std::min(l, lgN);
+  }
+  if (lgN <= most) return lgN;
+  auto passes = [&](int l) { return (lgN - l + per - 1) / per; };
+  int best = most;
+  for (int l = most - 1; l >= lo; --l)
+    if (passes(l) <= passes(best)) best = l;
   return best;
 }
 
 // sub_max: shared-memory sub-transform size for transforms longer than it (0:
-// d_sub_lg; the results do not depend on it, only where each butterfly runs)
+// sub_lg; the results do not depend on it, only where each butterfly runs)
 static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
   if (!is_pow2(n)) return set_err(MPFFT_EINVAL, "n=%lu is not a power of two", n);
   if (n > (1UL << 28)) return set_err(MPFFT_EUNSUPPORTED, "n=%lu too large", n);
   if (int e = device_ready()) return e;
   p->N = n;
-  p->tabs.N = (int)n;
   DSubTab &S = p->tabs.d;
   const int lgN = ilog2(n);
   S.N = (int)n;
-  S.lgT = lgN;
-  if (sub_max > 0) {
-    int l = 10;
-    while (l < 12 && (2 << l) <= sub_max) ++l;
-    if (lgN > l) S.lgT = l;
-  } else if (n > (unsigned long)kDSubMax) {
-    S.lgT = d_sub_lg(lgN);
-  }
+  S.lgT = sub_lg(lgN, 10, 12, 3, sub_max);
   const int T = 1 << S.lgT;
   S.nchunks = (int)(n / T);
   if (n > 16) {
@@ -1481,19 +1475,7 @@ static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
     S.slots[1] = S.slots[0];
     if (S.nchunks > 1) {
       if (int e = upload(p, leaf_slots(T / 2), &S.slots[1])) return e;
-      HostTree t;
-      walk(t, (int)n, 1, 0, 0, T);
-      std::vector<SrChunk> chunks(S.nchunks);
-      for (const Leaf &lf : t.leaves) {
-        SrChunk &c = chunks[lf.out / T];
-        c.chunk = lf.out / T;
-        if (lf.out % T == 0) c.sna = lf.sn;
-        else c.snb = lf.sn;
-      }
-      auto cls = [&](const SrChunk &c) { return ((c.sna % S.nchunks) + S.nchunks) % S.nchunks; };
-      std::stable_sort(chunks.begin(), chunks.end(),
-                       [&](const SrChunk &a, const SrChunk &b) { return cls(a) < cls(b); });
-      if (int e = upload(p, chunks, &S.chunks)) return e;
+      if (int e = upload(p, tree_chunks((int)n, T), &S.chunks)) return e;
     }
   }
   // twiddles exactly as the reference lut() (serial_d_fft6.c:52-62)
@@ -1714,27 +1696,23 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
   p->N = n;
   p->tier = tier;
   p->dd = tier == kTierDD;
-  p->tabs.N = (int)n;
-  const int T = (int)std::min<unsigned long>(n, (unsigned long)(sub_max > 0 ? sub_max : tier_sub_max(tier)));
-  {
-    HostTree t;
-    walk(t, (int)n, 1, 0, 0, T);
-    std::vector<SubRoot> roots;
-    for (const Leaf &lf : t.leaves) roots.push_back(SubRoot{lf.sn, lf.s, lf.out, lf.n});
-    p->tabs.nroots = (int)roots.size();
-    if (int e = upload(p, roots, &p->tabs.roots)) return e;
-    if (int e = build_tree(p->upper, n, T)) return e;
-    p->tabs.upper = p->upper.tabs;
+  TierTab &S = p->tabs.t;
+  const int lgN = ilog2(n), most = ilog2((unsigned long)tier_sub_max(tier));
+  S.N = (int)n;
+  S.lgT = sub_lg(lgN, most - 2, most, tier_pass_levels(tier), sub_max);
+  const int T = 1 << S.lgT;
+  S.nchunks = (int)(n / T);
+  if (n >= 8) {
+    if (int e = upload(p, tier_leaf_slots(T, 1 << tier_leaf_lg(tier)), &S.slots[0])) return e;
+    S.slots[1] = S.slots[0];
+    if (S.nchunks > 1) {
+      if (int e = upload(p, tier_leaf_slots(T / 2, 1 << tier_leaf_lg(tier)), &S.slots[1])) return e;
+      if (int e = upload(p, tree_chunks((int)n, T), &S.chunks)) return e;
+    }
   }
-  if (int e = build_sub(p, T, p->tabs.sub[0], 4)) return e;
-  if (T >= 2) {
-    if (int e = build_sub(p, T / 2, p->tabs.sub[1], 4)) return e;
-  } else {
-    p->tabs.sub[1] = p->tabs.sub[0];
-  }
-  const int K = tier == kTierQD ? 4 : tier == kTierDD ? 2 : 1;  // twiddle words
+  const int K = tier_tw_words(tier);
   const unsigned long q = std::max<unsigned long>(1, n / 4);
-  std::vector<double> w((size_t)2 * K * q);  // [cos words][sin words][k]
+  std::vector<double> w((size_t)2 * K * q);  // [word][cos, sin][k]
   parallel_for((long)q, 64, [&](long a, long b) {
     mpfr_t th, c, s;
     mpfr_init2(th, 360);
@@ -1746,10 +1724,11 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
       mpfr_div_ui(th, th, n, MPFR_RNDN);
       mpfr_sin_cos(s, c, th, MPFR_RNDN);
       for (int h = 0; h < K; ++h) {  // exact remainders at 320 bits
-        w[(size_t)h * q + k] = mpfr_get_d(c, MPFR_RNDN);
-        mpfr_sub_d(c, c, w[(size_t)h * q + k], MPFR_RNDN);
-        w[(size_t)(K + h) * q + k] = mpfr_get_d(s, MPFR_RNDN);
-        mpfr_sub_d(s, s, w[(size_t)(K + h) * q + k], MPFR_RNDN);
+        double *wc = &w[(size_t)(2 * h) * q + k], *ws = wc + q;
+        *wc = mpfr_get_d(c, MPFR_RNDN);
+        mpfr_sub_d(c, c, *wc, MPFR_RNDN);
+        *ws = mpfr_get_d(s, MPFR_RNDN);
+        mpfr_sub_d(s, s, *ws, MPFR_RNDN);
       }
     }
     mpfr_clear(th);
@@ -1757,19 +1736,18 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
     mpfr_clear(s);
     mpfr_free_cache();
   });
-  const double *dw = nullptr;
-  if (int e = upload(p, w, &dw)) return e;
-  for (int h = 0; h < K; ++h) {
-    p->tabs.tw_cos[h] = dw + (size_t)h * q;
-    p->tabs.tw_sin[h] = dw + (size_t)(K + h) * q;
-  }
-  p->tabs.wr = p->tabs.tw_cos[0];
-  p->tabs.wi = p->tabs.tw_sin[0];
-  if (K >= 2) {
-    p->tabs.wrl = p->tabs.tw_cos[1];
-    p->tabs.wil = p->tabs.tw_sin[1];
-  }
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
+  if (n >= 8) {  // the levels' twiddles, gathered from that table on the device (one allocation, see d_plan_init)
+    S.tw_len = n / 2 - 2;
+    double2 *d_tw = nullptr;
+    CUDA_TRY(cudaMalloc(&d_tw, S.tw_len * K * sizeof(double2) + w.size() * sizeof(double)));
+    p->dev_allocs.push_back(d_tw);
+    double *d_w = reinterpret_cast<double *>(d_tw + S.tw_len * K);
+    CUDA_TRY(cudaMemcpyAsync(d_w, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(tier_build_tw(d_w, K, (int)n, d_tw, p->stream));
+    CUDA_TRY(cudaStreamSynchronize(p->stream));
+    S.tw = d_tw;
+  }
   return MPFFT_OK;
 }
 
@@ -2381,7 +2359,7 @@ MPFFT_API int mpfft_dd_execute(mpfft_d_plan *plan, unsigned long batch, const do
   const double *src[4] = {xr_hi, xr_lo, xi_hi, xi_lo};
   for (int i = 0; i < 4; ++i) par_copy(plan->h_in + i * pl, src[i], pl);
   CUDA_TRY(cudaMemcpyAsync(plan->d_in, plan->h_in, 4 * pl * sizeof(double), cudaMemcpyHostToDevice, plan->stream));
-  CUDA_TRY(dd_run_transform(plan->tabs, plan->d_in, plan->d_out, (int)batch, d_scale(plan, flags), plan->stream));
+  CUDA_TRY(tier_run_transform(kTierDD, plan->tabs, plan->d_in, plan->d_out, (int)batch, d_scale(plan, flags), plan->stream));
   CUDA_TRY(cudaMemcpyAsync(plan->h_out, plan->d_out, 4 * pl * sizeof(double), cudaMemcpyDeviceToHost, plan->stream));
   CUDA_TRY(cudaStreamSynchronize(plan->stream));
   double *dst[4] = {yr_hi, yr_lo, yi_hi, yi_lo};
@@ -2400,7 +2378,7 @@ MPFFT_API int mpfft_dd_execute_device(mpfft_d_plan *plan, unsigned long batch, c
   const char *a = (const char *)d_in, *b = (const char *)d_out;
   if (a < b + bytes && b < a + bytes) return set_err(MPFFT_EINVAL, "input and output buffers overlap");
   const bool inv = (flags & MPFFT_INVERSE) != 0;
-  CUDA_TRY(dd_run_transform(plan->tabs, d_in, d_out, (int)batch, d_scale(plan, flags), (cudaStream_t)stream, inv,
+  CUDA_TRY(tier_run_transform(kTierDD, plan->tabs, d_in, d_out, (int)batch, d_scale(plan, flags), (cudaStream_t)stream, inv,
                             inv));
   return set_err(MPFFT_OK, "");
 }

@@ -52,35 +52,6 @@ struct MpDeviceTables : TreeTables {
                 // kTcMinLimbs limbs, 2 from kTcForceMinLimbs limbs
 };
 
-// Schedule of one shared-memory sub-transform of size `size` (FP64 tier):
-// perm[j] = the position that element j of the sub-transform's input sequence
-// takes (the DIT input order), then the leaves (n <= 16, in place over
-// positions [out, out+n)) and the levels of the size-`size` tree.
-struct SubSchedule {
-  int size = 0;
-  const int *perm = nullptr;
-  int nleaves = 0;
-  int nleaf16 = 0, nleaf8 = 0;   // leaves are sorted: 16-point, 8-point, then smaller
-  const Leaf *leaves = nullptr;  // .sn/.s unused: inputs are already in place
-  int nlevels = 0;
-  int level_n[kMaxLevels] = {};
-  int level_start[kMaxLevels] = {};
-  int level_count[kMaxLevels] = {};
-  const int *node_off = nullptr;
-  // for levels lv and lv+1 run in one pass (each node of size level_n[lv+1]
-  // with its first child): the nodes of size level_n[lv] that are not a first
-  // child, at pair_nodes + pair_start[lv] (pair_count[lv] of them)
-  const int *pair_nodes = nullptr;
-  int pair_start[kMaxLevels] = {};
-  int pair_count[kMaxLevels] = {};
-};
-
-// root of a shared-memory sub-transform: input elements x[(sn + j*s)] (j = 0
-// wrapped to sn + N when sn < 0), outputs y[out .. out+size)
-struct SubRoot {
-  int sn, s, out, size;
-};
-
 // FP64 base-case constants
 struct DConst {
   double c8 = 0, c16a = 0, c16b = 0, c16c = 0, c16d = 0;
@@ -108,29 +79,31 @@ struct DSubTab {
   DConst K;
 };
 
+// Base cases of the output positions of one slot of a tier's sub-transform.
+// Eight positions: a leaf of 4 points (input in[0]) and another (in[1]) or two
+// of 2 points (in[1], in[2]); four positions: a leaf of 4 (in[0]) or two of 2.
+struct TierLeafSlot {
+  int m, in[3];
+};
+
+// compensated tiers (float_tiers.cuh): chunks of T = 2^lgT points run in shared memory
+struct TierTab {
+  int N = 0, lgT = 0;
+  int nchunks = 0;                        // N/T
+  const TierLeafSlot *slots[2] = {};      // base cases of a T- and a T/2-point tree
+  const SrChunk *chunks = nullptr;        // by input class
+  const double2 *tw = nullptr;            // (cos, sin) per level n = 8 .. N, tier_level_tw; planes by word
+  size_t tw_len = 0;                      // entries of a plane
+};
+
 struct DDeviceTables {
-  int N = 0;
-  DSubTab d;  // FP64 plans; the fields below: compensated tiers
-  const double *wr = nullptr;  // [N/4] cos(2 pi k/N)
-  const double *wi = nullptr;  // [N/4] sin(2 pi k/N)
-  const double *wrl = nullptr, *wil = nullptr;  // double-double plans: low parts of wr, wi
-  // compensated tiers (float_tier_kernels.cu): the words of cos and sin of
-  // 2 pi k/N, k < N/4 (double-double: 2, quad-double: 4, float-float: 1 double)
-  const double *tw_cos[4] = {}, *tw_sin[4] = {};
-  // shared-memory sub-transforms (sizes T and T/2) ...
-  int nroots = 0;
-  const SubRoot *roots = nullptr;
-  SubSchedule sub[2];
-  // ... and the levels above them, in global memory
-  TreeTables upper;
+  DSubTab d;   // FP64 plans
+  TierTab t;   // compensated tiers
 };
 
 constexpr int kMaxDevices = 64;
 constexpr int kDSubMax = 4096;  // FP64: most points a CTA holds in shared memory (64 KB)
 constexpr int kDSubMin = 64;    // FP64: smallest sub-transform of a longer transform
-constexpr int kDDSubMax = 2048; // double-double: largest shared-memory sub-transform (64 KB)
-constexpr int kQDSubMax = 1024; // quad-double (64 KB)
-constexpr int kFFSubMax = 4096; // float-float (64 KB)
 // compensated floating-point tiers (float_tier_kernels.cu)
 enum { kTierDD = 0, kTierQD = 1, kTierFF = 2 };
 
@@ -250,9 +223,6 @@ cudaError_t d_build_level_tw(const double *wr, const double *wi, int N, double2 
 // planes exchanged (both: the unscaled inverse, swap(FFT(swap(x))))
 cudaError_t d_run_transform(const DDeviceTables &T, const double *in, double *out, int B, double scale,
                             cudaStream_t s, bool swap_in = false, bool swap_out = false);
-// double-double tier (dd_kernels.cu); layout word (c, h, b, p) at ((c*2 + h)*B + b)*N + p
-cudaError_t dd_run_transform(const DDeviceTables &T, const double *in, double *out, int B, double scale,
-                             cudaStream_t s, bool swap_in = false, bool swap_out = false);
 // any compensated tier; layout word (c, h, b, p) at ((c*K + h)*B + b)*N + p with
 // K = tier_words(tier) words of tier_word_bytes(tier) bytes per real component
 cudaError_t tier_run_transform(int tier, const DDeviceTables &T, const void *in, void *out, int B, double scale,
@@ -260,6 +230,12 @@ cudaError_t tier_run_transform(int tier, const DDeviceTables &T, const void *in,
 int tier_words(int tier);
 size_t tier_word_bytes(int tier);
 int tier_sub_max(int tier);
+int tier_tw_words(int tier);     // words of a twiddle's cos (and of its sin)
+int tier_pass_levels(int tier);  // levels per pass
+int tier_leaf_lg(int tier);      // lg of the positions of a base-case slot
+// tw[h*len + level entry] = (cos, sin) word h of 2 pi k/n for every level n = 8
+// .. N, from w[(2h + part)*q + k'] of the N-point table (q = N/4)
+cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaStream_t s);
 // split step of the FP64 real transforms (n = 2M real points), d_kernels.cu
 cudaError_t d_real_split(bool forward, const double *in, double *out, int M, int B, const double *wc,
                          const double *ws, double scale, cudaStream_t s);

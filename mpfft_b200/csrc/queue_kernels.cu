@@ -128,36 +128,45 @@ __global__ void __launch_bounds__(256, 2) d_queue_kernel(const QueueItem *__rest
 // ---------------------------------------------------------------------------
 // compensated tiers: the same pattern
 // ---------------------------------------------------------------------------
+template <class NT, int R>
+__device__ __forceinline__ void tier_queue_upper(const TierTab &S, typename NT::W *out, int lgu, int cols, double scale) {
+  for (int t = threadIdx.x; t < cols; t += blockDim.x)
+    tier_upper_column<NT, R>(out, S, 1, lgu, 0, t >> lgu, t & ((1 << lgu) - 1), scale, false);
+}
+
 template <class NT>
 __global__ void __launch_bounds__(256) tier_queue_kernel(const QueueItem *__restrict__ items, int nitems, int *head,
                                                          double scale) {
-  extern __shared__ __align__(16) unsigned char tq_smem[];
-  typename NT::W *sm = reinterpret_cast<typename NT::W *>(tq_smem);
+  extern __shared__ __align__(16) double2 tq_smem[];
   __shared__ int slot;
   for (int i; (i = queue_next(head, &slot)) < nitems;) {
     const QueueItem it = items[i];
-    const DDeviceTables &T = it.tab->ft;
-    const auto *in = static_cast<const typename NT::W *>(it.in);
+    const TierTab S = it.tab->ft.t;
     auto *out = static_cast<typename NT::W *>(it.out);
-    TierTw tw{};
-    for (int h = 0; h < 4; ++h) {
-      tw.c[h] = T.tw_cos[h];
-      tw.s[h] = T.tw_sin[h];
+    const int nl = 31 - __clz(S.nchunks);
+    TierArgs<NT> A{static_cast<const typename NT::W *>(it.in), out, 1, 0, 0, 1, NT::kLevels, scale, nl == 0, false, false};
+    if (S.N < 8) {
+      tier_tiny<NT>(S, A);
+      continue;
     }
-    const bool final_sub = T.upper.nlevels == 0;
-    for (int r = 0; r < T.nroots; ++r) {
-      __syncthreads();
-      tier_sub_instances<NT, false>(in, out, T.N, 1, 0, 1, T.roots[r], T.sub[0], T.sub[1], tw,
-                                    final_sub ? scale : 1.0, 0, 0, sm);
+    if (nl == 0) {
+      tier_sub_transform<NT, true>(S, A, tq_smem);
+      continue;
     }
-    for (int lv = 0; lv < T.upper.nlevels; ++lv) {
+    for (A.c0 = 0; A.c0 < S.nchunks; ++A.c0) {
+      __syncthreads();  // shared memory of the previous chunk is free
+      tier_sub_transform<NT, false>(S, A, tq_smem);
+    }
+    const int step = tier_upper_levels(nl, NT::kLevels);
+    for (int done = 0; done < nl;) {
       __syncthreads();
-      const int n = T.upper.level_n[lv], q = n >> 2;
-      const int total = T.upper.level_count[lv] * q;
-      const int *nodes = T.upper.node_off + T.upper.level_start[lv];
-      const double sc = lv == T.upper.nlevels - 1 ? scale : 1.0;
-      for (int t = threadIdx.x; t < total; t += blockDim.x)
-        tier_level_one<NT>(out, T.N, 1, n, nodes[t / q], t % q, 0, tw, sc, 0);
+      const int r = min(step, nl - done), lgu = S.lgT + done - 1, cols = S.N >> (r + 1);
+      const double sc = done + r == nl ? scale : 1.0;
+      constexpr int R2 = NT::kLevels >= 2 ? 2 : 1, R3 = NT::kLevels >= 3 ? 3 : 1;
+      if (r == 3) tier_queue_upper<NT, R3>(S, out, lgu, cols, sc);
+      else if (r == 2) tier_queue_upper<NT, R2>(S, out, lgu, cols, sc);
+      else tier_queue_upper<NT, 1>(S, out, lgu, cols, sc);
+      done += r;
     }
   }
 }
@@ -165,7 +174,7 @@ __global__ void __launch_bounds__(256) tier_queue_kernel(const QueueItem *__rest
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr size_t kQueueSmemBytes = 64 * 1024;  // FP64 (4096 points) and every tier (64 KB planes)
+constexpr size_t kQueueSmemBytes = 64 * 1024 + kOrderBytes;  // FP64 (4096 points) and every tier (64 KB planes)
 
 template <int L>
 static const void *mp_queue_fn() {

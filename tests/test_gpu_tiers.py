@@ -164,3 +164,36 @@ def test_float_tier_out_of_window_runs_on_limbs(M, orc):
     L = O.lib()
     assert L.orc_mp_count_diff(yr.ptr, zr.ptr, n * batch) == 0
     assert L.orc_mp_count_diff(yi.ptr, zi.ptr, n * batch) == 0
+
+
+@pytest.mark.parametrize("tier", ["ff", "dd", "qd"])
+@pytest.mark.parametrize("n,batch", [(4, 300), (8, 257), (16, 3), (32, 600), (128, 17), (256, 9), (512, 5), (1024, 3),
+                                     (2048, 3), (8192, 2), (32768, 1)])
+def test_tier_register_passes_inverse_scaled(M, orc, tier, n, batch):
+    """Every chain of base cases and register passes, partly filled CTAs, planes
+    exchanged and scaled: the scaled inverse against the oracle's transform of
+    the exchanged input (the swap identity), within the tier's bound."""
+    import torch
+
+    O = orc
+    bits, prec = {"ff": (44, 96), "dd": (104, 212), "qd": (206, 424)}[tier]
+    plan = M.MultiwordPlan(n, tier)
+    K, fl = plan.words, plan.word_bytes == 4
+    xr, xi = O.mp_pair(n, {"ff": 48, "dd": 106, "qd": 212}[tier])
+    O.fill_uniform(xr, xi, n + K)
+    one = np.stack([_words(O, xr, K, fl), _words(O, xi, K, fl)])  # [2][K][n]
+    x = np.repeat(one[:, :, None, :], batch, axis=2)
+    x[:, :, : batch // 2] *= -1  # other signals than the last
+    d_in = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    d_out = torch.full_like(d_in, float("nan"))
+    plan.execute_device(batch, d_in.data_ptr(), d_out.data_ptr(), scaled=True, inverse=True,
+                        stream=torch.cuda.current_stream().cuda_stream)
+    y = d_out.cpu().numpy()
+    if batch > 1:
+        assert np.array_equal(y[:, :, 0], -y[:, :, -1])
+    sr, si = _from_words(O, one[0], prec), _from_words(O, one[1], prec)
+    dr, di = O.mp_pair(n, prec)
+    O.MpFFT(n, prec)(si, sr, di, dr)  # exchanged in, exchanged out: the unscaled inverse
+    gr, gi = _from_words(O, y[0, :, -1] * n, prec), _from_words(O, y[1, :, -1] * n, prec)
+    e = O.mp_errors(gr, gi, dr, di)["log2_rel"]
+    assert e <= math.log2(8 * max(1.0, math.log2(n))) - bits, e
