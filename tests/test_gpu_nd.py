@@ -134,3 +134,23 @@ def test_d_nd_bitexact_vs_axis_by_axis_reference(M, orc, dims, batch):
     # and within rounding of numpy's transform
     ref = np.fft.fftn(xr + 1j * xi, axes=tuple(range(1, len(dims) + 1)))
     assert np.max(np.abs(yr + 1j * yi - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("dims", [(2, 128), (128, 2), (16, 256), (64, 32), (2, 4, 256), (1, 512)])
+@pytest.mark.parametrize("batch", [1, 2])
+def test_mp_nd_word_transpositions_equal_wider_elements(M, orc, dims, batch):
+    """One or two signals are transposed as elements of one or two words, by
+    tiles of 32 rows x 128 (64) columns (fewer where the axis is shorter); the
+    same signals among three are elements of three words.  Bit for bit."""
+    O = orc
+    L = O.lib()
+    n, p = _prod(dims), 100
+    xr, xi = O.mp_pair(3 * n, p)
+    O.fill_uniform(xr, xi, 23)
+    plan = M.MpPlanND(dims, p)
+    yr, yi = O.mp_pair(3 * n, p)
+    plan.execute(3, xr.ptr, xi.ptr, yr.ptr, yi.ptr)
+    zr, zi = O.mp_pair(batch * n, p)
+    plan.execute(batch, xr.ptr, xi.ptr, zr.ptr, zi.ptr)
+    assert L.orc_mp_count_diff(zr.ptr, yr.ptr, batch * n) == 0
+    assert L.orc_mp_count_diff(zi.ptr, yi.ptr, batch * n) == 0

@@ -175,3 +175,23 @@ def test_queue_long_limb_signals_run_as_groups(M, orc):
     O.MpFFT(n, 2 * p)(xr, xi, wr, wi)
     e = O.mp_errors(outs[0][0], outs[0][1], wr, wi)["log2_rel"]
     assert e <= O.mp_bound_log2(n, p), (e, O.mp_bound_log2(n, p))
+
+
+@pytest.mark.parametrize("count", [1, 3, 31, 33, 65])
+def test_queue_groups_of_ragged_sizes(M, orc, count):
+    """A group's signals are interleaved and taken apart by tiles of 32 signals;
+    a group of any size gives every signal the bits of a batched transform."""
+    O = orc
+    L = O.lib()
+    n, p = 4096, 64
+    xr, xi = O.mp_pair(n * count, p)
+    O.fill_uniform(xr, xi, 31)
+    at = [32 * n * i for i in range(count)]
+    plan = M.BatchPlan([n] * count, [p] * count, float_tiers=False)
+    assert [q["signals"] for q in plan.queues() if q["threads"] == 0] == [count]
+    yr, yi = O.mp_pair(n * count, p)
+    plan.execute([xr.ptr + o for o in at], [xi.ptr + o for o in at], [yr.ptr + o for o in at], [yi.ptr + o for o in at])
+    zr, zi = O.mp_pair(n * count, p)
+    M.MpPlan(n, p, float_tiers=False).execute(count, xr.ptr, xi.ptr, zr.ptr, zi.ptr)
+    assert L.orc_mp_count_diff(yr.ptr, zr.ptr, n * count) == 0
+    assert L.orc_mp_count_diff(yi.ptr, zi.ptr, n * count) == 0
