@@ -2909,7 +2909,7 @@ MPFFT_API int mpfft_batch_plan_create(mpfft_batch_plan **plan, unsigned long cou
       t.N = (int)s.n;
       if (fam == kQueueLimbs) {
         t.tree = s.mp->tabs;
-        t.tw = s.mp->tabs.tw;
+        t.twp = s.mp->tabs.twp;
         t.dneg = s.mp->tabs.dneg;
       }
       bp->tabs.push_back(t);

@@ -152,26 +152,24 @@ __device__ __forceinline__ void combine(uint32_t *u0, uint32_t *u1, uint32_t *zp
 // combine: the products of the Z+ slots (zp) and Z- slots (zm) by w^k and
 // w^-k, merged and stored back into the slots swapped (m.r in the imaginary
 // slot, m.i in the real one).  n: the node size (q = n/4); P: this thread's
-// slot for the side's first product (words ps apart); Twp: the CTA's packed
-// twiddles (kPackedTw only).  The merged products are stored with L2 priority
+// slot for the side's first product (words ps apart); twp: packed twiddles of
+// all k ([k][cos, cos+sin, |cos-sin|][Lp]: a row is read four limbs per load, for
+// one row a product instead of L strided words; N=1024, batch 2048, 33 limbs: 2357
+// -> 2288 us, 65536 points, batch 24, 34 limbs: 3608 -> 3494 us).  The merged products are stored with L2 priority
 // evict_last (a fused thread of mp_level_pair_kernel reads them back only
 // after two more butterflies).  mp_bfly_one below spells out the same steps
 // inline (its register allocation at 33 limbs spills less that way); the
 // kernels built on each are checked to be bit-identical.
-template <int L, bool kPackedTw>
+template <int L>
 __device__ __forceinline__ void mp_bfly_steps(uint32_t *zp, uint32_t *zm, size_t plane, size_t cim, int N, int n,
-                                              int k, const uint32_t *__restrict__ tw,
-                                              const uint8_t *__restrict__ dneg, int tws, uint32_t *P, size_t ps,
-                                              const uint32_t *Twp) {
+                                              int k, const uint32_t *__restrict__ twp,
+                                              const uint8_t *__restrict__ dneg, int tws, uint32_t *P, size_t ps) {
   const int q = n >> 2;
-  const size_t tplane = (size_t)(N >> 2) * tws;  // twiddle limb-plane stride
   const int kn = k * (N / n) * tws;
-  const uint32_t *wr = tw + kn;                           // cos
-  const uint32_t *ws = tw + (size_t)L * tplane + kn;      // cos + sin
-  const uint32_t *wd = tw + (size_t)2 * L * tplane + kn;  // |cos - sin|
   const bool special = (2 * k == q);
   const bool dn = special ? false : (dneg[kn] != 0);
   constexpr int Lp = (L + 3) & ~3;  // packed twiddle stride: 16-byte aligned rows
+  const uint32_t *row = twp + (size_t)kn * (3 * Lp);
   uint32_t X[L];
 #pragma unroll 1
   for (int st_ = 0; st_ < 6; ++st_) {
@@ -179,7 +177,7 @@ __device__ __forceinline__ void mp_bfly_steps(uint32_t *zp, uint32_t *zm, size_t
     const int step = st_ - 3 * side;
     uint32_t *zr = side ? zm : zp;
     uint32_t *zi = zr + cim;
-    const uint32_t *pa = zr, *pb = nullptr, *w = wr;
+    const uint32_t *pa = zr, *pb = nullptr;
     int wsel = 0;  // packed twiddle row: 0 cos, 1 cos+sin, 2 |cos-sin|
     bool sub = false, negx = false, mul = true;
     int sp = 0;
@@ -190,13 +188,11 @@ __device__ __forceinline__ void mp_bfly_steps(uint32_t *zp, uint32_t *zm, size_t
     } else if (!special) {
       if (step == 1) {
         pa = zi;
-        w = wd;
         wsel = 2;
         negx = dn ^ (side == 0);
         sp = 1;
         dst = zi;
       } else {
-        w = ws;
         wsel = 1;
         negx = (side == 0);
         sp = side ? -1 : 1;
@@ -216,8 +212,7 @@ __device__ __forceinline__ void mp_bfly_steps(uint32_t *zp, uint32_t *zm, size_t
     }
     if (mul) {
       ld_addsub<L>(X, pa, pb, plane, sub);
-      if (kPackedTw) mul_tw<L, true>(X, Twp + wsel * Lp, 0);
-      else mul_tw<L>(X, w, tplane);
+      mul_tw<L, true>(X, row + wsel * Lp, 0);
     } else {
 #pragma unroll
       for (int i = 0; i < L; ++i) X[i] = 0;
@@ -236,11 +231,11 @@ __device__ __forceinline__ void mp_bfly_steps(uint32_t *zp, uint32_t *zm, size_t
 
 // One butterfly k of one signal b (the body of mp_level_kernel): the node of
 // size n at output offset off.  P: this thread's slot for the side's first
-// product (words ps apart); Twp: the CTA's packed twiddles (kPackedTw only).
-template <int L, bool kPackedTw>
+// product (words ps apart); twp as in mp_bfly_steps.
+template <int L>
 __device__ __forceinline__ void mp_bfly_one(uint32_t *__restrict__ y, int N, int B, int b, int n, int off, int k,
-                                            const uint32_t *__restrict__ tw, const uint8_t *__restrict__ dneg,
-                                            int tws, uint32_t *P, size_t ps, const uint32_t *Twp) {
+                                            const uint32_t *__restrict__ twp, const uint8_t *__restrict__ dneg,
+                                            int tws, uint32_t *P, size_t ps) {
   const int q = n >> 2;
   const size_t plane = (size_t)N * B;
   const size_t cim = (size_t)L * plane;
@@ -253,14 +248,11 @@ __device__ __forceinline__ void mp_bfly_one(uint32_t *__restrict__ y, int N, int
     combine<L>(u0, u1, zp, zm, plane, cim, false);
     return;
   }
-  const size_t tplane = (size_t)(N >> 2) * tws;  // twiddle limb-plane stride
   const int kn = k * (N / n) * tws;
-  const uint32_t *wr = tw + kn;                           // cos
-  const uint32_t *ws = tw + (size_t)L * tplane + kn;      // cos + sin
-  const uint32_t *wd = tw + (size_t)2 * L * tplane + kn;  // |cos - sin|
   const bool special = (2 * k == q);
   const bool dn = special ? false : (dneg[kn] != 0);
   constexpr int Lp = (L + 3) & ~3;  // packed twiddle stride: 16-byte aligned rows
+  const uint32_t *row = twp + (size_t)kn * (3 * Lp);
   uint32_t X[L];
 #pragma unroll 1
   for (int st_ = 0; st_ < 6; ++st_) {
@@ -268,7 +260,7 @@ __device__ __forceinline__ void mp_bfly_one(uint32_t *__restrict__ y, int N, int
     const int step = st_ - 3 * side;
     uint32_t *zr = side ? zm : zp;
     uint32_t *zi = zr + cim;
-    const uint32_t *pa = zr, *pb = nullptr, *w = wr;
+    const uint32_t *pa = zr, *pb = nullptr;
     int wsel = 0;  // packed twiddle row: 0 cos, 1 cos+sin, 2 |cos-sin|
     bool sub = false, negx = false, mul = true;
     int sp = 0;
@@ -279,13 +271,11 @@ __device__ __forceinline__ void mp_bfly_one(uint32_t *__restrict__ y, int N, int
     } else if (!special) {
       if (step == 1) {
         pa = zi;
-        w = wd;
         wsel = 2;
         negx = dn ^ (side == 0);
         sp = 1;
         dst = zi;
       } else {
-        w = ws;
         wsel = 1;
         negx = (side == 0);
         sp = side ? -1 : 1;
@@ -305,8 +295,7 @@ __device__ __forceinline__ void mp_bfly_one(uint32_t *__restrict__ y, int N, int
     }
     if (mul) {
       ld_addsub<L>(X, pa, pb, plane, sub);
-      if (kPackedTw) mul_tw<L, true>(X, Twp + wsel * Lp, 0);
-      else mul_tw<L>(X, w, tplane);
+      mul_tw<L, true>(X, row + wsel * Lp, 0);
     } else {
 #pragma unroll
       for (int i = 0; i < L; ++i) X[i] = 0;

@@ -152,18 +152,10 @@ __global__ void __launch_bounds__(128) mp_leaf_small_kernel(const uint32_t *__re
 //                                   -> re slot
 // so m.r ends in the imaginary slot and m.i in the real slot ("swapped").
 
-// Batches that are a multiple of the CTA size give every CTA one (node, k):
-// up to 31 limbs the CTA then stages its three twiddles in shared memory once
-// and the products read them four limbs per load (measured at N=1024, batch
-// 2048: +4.6 % at 9 limbs, +3.1 % at 17, +0.4 to +2.2 % at 31; -0.7 % at 33,
-// where the 128-register product already spills, so the larger limb counts
-// keep the per-row global loads).
-constexpr int kPackedTwiddleMaxLimbs = 31;
-
-template <int L, bool kPackedTw>
+template <int L>
 __global__ void __launch_bounds__(128, level_min_blocks<L>()) mp_level_kernel(uint32_t *__restrict__ y, int N, int B, int n,
                                                           const int *__restrict__ node_off, int nnodes,
-                                                          const uint32_t *__restrict__ tw,
+                                                          const uint32_t *__restrict__ twp,
                                                           const uint8_t *__restrict__ dneg, int tws) {
   __shared__ uint32_t Ps[L * 128];
   const int q = n >> 2;
@@ -173,18 +165,7 @@ __global__ void __launch_bounds__(128, level_min_blocks<L>()) mp_level_kernel(ui
   const long long r = t / B;
   const int k = (int)(r % q);
   const int off = node_off[r / q];
-  constexpr int Lp = (L + 3) & ~3;
-  __shared__ __align__(16) uint32_t Tw[kPackedTw ? 3 * Lp : 4];
-  if (kPackedTw && k != 0) {  // cos, cos+sin, |cos-sin| of this CTA's k (every thread of the CTA has it)
-    const size_t tplane = (size_t)(N >> 2) * tws;
-    const int kn = k * (N / n) * tws;
-    for (int e = threadIdx.x; e < 3 * L; e += blockDim.x) {
-      const int sel = e / L, j = e - sel * L;
-      Tw[sel * Lp + j] = tw[(size_t)(sel * L + j) * tplane + kn];
-    }
-    __syncthreads();
-  }
-  mp_bfly_one<L, kPackedTw>(y, N, B, b, n, off, k, tw, dneg, tws, Ps + threadIdx.x, blockDim.x, Tw);
+  mp_bfly_one<L>(y, N, B, b, n, off, k, twp, dneg, tws, Ps + threadIdx.x, blockDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -230,11 +211,11 @@ struct CombineChains {
 // Limb counts up to which combine_pair's limb loop is unrolled; above, the
 // unrolled loop's register demand next to the 128-register product costs more
 // than it saves, and the rolled loop reads the Z slots through ld_hint (kept
-// in program order; 33 limbs 3.02 -> 2.91 ms, 9 and 17 limbs 6 % slower that
-// way).  N=1024, batch 2048, ms per transform batch, unrolled / rolled with
-// plain loads: 9 limbs 0.517 / 0.601, 17 limbs 1.091 / 1.186, 25 limbs 1.886 /
-// 1.886, 29 limbs 2.479 / 2.337, 33 limbs 3.265 / 3.010, 34 limbs 3.489 / 3.279.
-constexpr int kPairUnrollMaxLimbs = 25;
+// in program order).  N=1024, batch 2048, ms per transform batch, unrolled /
+// rolled: 9 limbs 0.438 / 0.456, 17 limbs 0.914 / 0.932, 21 limbs 1.194 / 1.184,
+// 25 limbs 1.501 / 1.467, 29 limbs 2.093 / 1.922, 33 limbs 2.353 / 2.298, 34 limbs
+// 2.465 / 2.386.
+constexpr int kPairUnrollMaxLimbs = 20;
 
 // One limb of the three L-combines of a fused thread; p: limb i of position k
 // of the pair's node Y (word stride qB = q*B between the positions k + j*q).
@@ -282,8 +263,8 @@ __device__ __forceinline__ void combine_pair(uint32_t *p, size_t qB, size_t plan
 // CTAs per SM of mp_level_pair_kernel: from 31 limbs three (up to 170
 // registers, no spills) instead of the one-level kernel's four, whose
 // 128-register product spills (N=1024, batch 2048, ms per batch, four / three
-// CTAs: 21 limbs 1.435 / 1.519, 25 1.837 / 1.929, 29 2.299 / 2.319, 31 2.706 /
-// 2.638, 33 2.913 / 2.833, 34 3.257 / 3.005).
+// CTAs: 21 limbs 1.194 / 1.297, 25 1.501 / 1.605, 29 1.922 / 1.928, 31 2.163 /
+// 2.107, 33 2.500 / 2.298, 34 2.674 / 2.386).
 template <int L>
 constexpr int pair_min_blocks() {
   return L >= 31 ? 3 : level_min_blocks<L>();
@@ -292,7 +273,7 @@ constexpr int pair_min_blocks() {
 template <int L>
 __global__ void __launch_bounds__(128, pair_min_blocks<L>()) mp_level_pair_kernel(
     uint32_t *__restrict__ y, int N, int B, int n, const int *__restrict__ ynodes, int ny,
-    const int *__restrict__ unodes, int nu, const uint32_t *__restrict__ tw, const uint8_t *__restrict__ dneg,
+    const int *__restrict__ unodes, int nu, const uint32_t *__restrict__ twp, const uint8_t *__restrict__ dneg,
     int tws) {
   __shared__ uint32_t Ps[L * 128];
   const int q = n >> 2;
@@ -316,8 +297,8 @@ __global__ void __launch_bounds__(128, pair_min_blocks<L>()) mp_level_pair_kerne
     const int kk = j == 2 ? k + q : k;
     if (kk == 0) continue;
     const int zs = j == 0 ? 2 : (j == 1 ? 4 : 5);  // Z+ slot at zs*q, Z- at (zs+1)*q or (zs+2)*q
-    mp_bfly_steps<L, false>(p + (size_t)zs * qB, p + (size_t)(j == 0 ? 3 : zs + 2) * qB, plane, cim, N,
-                            j == 0 ? n : 2 * n, kk, tw, dneg, tws, Ps + threadIdx.x, blockDim.x, nullptr);
+    mp_bfly_steps<L>(p + (size_t)zs * qB, p + (size_t)(j == 0 ? 3 : zs + 2) * qB, plane, cim, N, j == 0 ? n : 2 * n, kk,
+                     twp, dneg, tws, Ps + threadIdx.x, blockDim.x);
   }
   if (fused) combine_pair<L>(p, qB, plane, cim, k != 0);
   else combine<L>(p, p + qB, p + 2 * qB, p + 3 * qB, plane, cim, k != 0);
@@ -336,18 +317,19 @@ __global__ void __launch_bounds__(128, pair_min_blocks<L>()) mp_level_pair_kerne
 // after a second barrier eight threads run the L-combine, one output
 // component each (three loads per limb, all limbs in flight at once, instead
 // of eight per limb on one thread: one signal at N=1024, P=1024 5.3k -> 7.7k
-// transforms/s, 16 signals 71k -> 107k).  The same modular sums of the same
+// transforms/s, 16 signals 71k -> 107k).  Twiddles are read from the packed rows
+// (8 signals, N=1024, 17 limbs: planes 38.3 us, rows 37.4).  The same modular sums of the same
 // operands, so the results are bit-identical.
 
 // Step st (0..5) of a twiddled butterfly: side st/3 (0: Z+ at zp, 1: Z- at
 // zm), step st%3.  X = pa (+ or - pb when pb is set), X *= the twiddle whose
-// first limb w points at (cos, cos+sin or |cos-sin|) when mul, else X = 0;
+// row w points at (cos, cos+sin or |cos-sin|) when mul, else X = 0;
 // then either X becomes the side's first product P (dst null) or
 // dst = (negx ? -X : X) + sp * P.  This is the step table of mp_level_kernel,
 // which spells it out inline in its step loop (the struct form measured 4 %
 // slower there); the two kernels are checked to be bit-identical.
 struct BflyStep {
-  const uint32_t *pa, *pb, *w;  // w: the twiddle row's first limb (planes)
+  const uint32_t *pa, *pb, *w;  // w: the twiddle row's first limb
   uint32_t *dst;
   int sp;
   bool sub, negx, mul;
@@ -435,8 +417,9 @@ __device__ __forceinline__ void combine_one(int o, bool valid, uint32_t *u0, uin
 template <int L>
 __global__ void __launch_bounds__(8 * kSmallBflies) mp_level_small_kernel(uint32_t *__restrict__ y, int N, int B,
                                                                           int n, const int *__restrict__ node_off,
-                                                                          int nnodes, const uint32_t *__restrict__ tw,
+                                                                          int nnodes, const uint32_t *__restrict__ twp,
                                                                           const uint8_t *__restrict__ dneg, int tws) {
+  constexpr int Lp = (L + 3) & ~3;
   __shared__ uint32_t Qs[kSmallBflies * 6 * L];  // [butterfly][step][limb]
   pdl_release();
   const int lb = threadIdx.x >> 3, st_ = threadIdx.x & 7;  // steps 0..5; all 8 in the combine
@@ -459,17 +442,16 @@ __global__ void __launch_bounds__(8 * kSmallBflies) mp_level_small_kernel(uint32
     zp = u0 + (size_t)2 * q * B;
     zm = u0 + (size_t)3 * q * B;
     if (k != 0 && st_ < 6) {
-      const size_t tplane = (size_t)(N >> 2) * tws;
       const int kn = k * (N / n) * tws;
       const bool special = (2 * k == q);
       const bool dn = special ? false : (dneg[kn] != 0);
-      S = bfly_step(st_, special, dn, zp, zm, cim, tw + kn, tw + (size_t)L * tplane + kn,
-                    tw + (size_t)2 * L * tplane + kn);
+      const uint32_t *row = twp + (size_t)kn * (3 * Lp);
+      S = bfly_step(st_, special, dn, zp, zm, cim, row, row + Lp, row + 2 * Lp);
       pdl_wait();
       uint32_t X[L];
       if (S.mul) {
         ld_addsub<L>(X, S.pa, S.pb, plane, S.sub);
-        mul_tw<L>(X, S.w, tplane);
+        mul_tw<L, true>(X, S.w, 0);
       } else {
 #pragma unroll
         for (int i = 0; i < L; ++i) X[i] = 0;
@@ -503,7 +485,9 @@ __global__ void __launch_bounds__(8 * kSmallBflies) mp_level_small_kernel(uint32
 // shared memory; every global input a warp needs (its step's operands, its
 // output's U and, without twiddle, the Z slots) is loaded before the first
 // barrier and every output is stored after the second, so the in-place update
-// is safe.  The same sums of the same operands: bit-identical.
+// is safe.  The same sums of the same operands: bit-identical.  The twiddles
+// come from their limb planes: read from the packed rows the same kernel takes
+// longer (one signal of N=1024, 17 limbs 26.4 -> 31.1 us, 25 limbs 35.2 -> 40.2).
 constexpr int kWarpBflyThreads = 256;
 
 template <int L>
@@ -705,7 +689,7 @@ static cudaError_t run_transform(const MpDeviceTables &T, const uint32_t *in, ui
       timer.begin();
       mp_level_pair_kernel<L><<<(unsigned)((threads + lthreads - 1) / lthreads), lthreads, 0, s>>>(
           out, T.N, B, n, T.node_off + T.level_start[lv + 1], T.level_count[lv + 1],
-          T.pair_nodes + T.pair_start[lv], T.pair_count[lv], T.tw, T.dneg, T.tws);
+          T.pair_nodes + T.pair_start[lv], T.pair_count[lv], T.twp, T.dneg, T.tws);
       timer.end();
       timer.none();
       ++lv;
@@ -721,13 +705,10 @@ static cudaError_t run_transform(const MpDeviceTables &T, const uint32_t *in, ui
     else if (total < kSmallLevelButterflies)
       e = launch_pdl(pdl, mp_level_small_kernel<L>, (unsigned)((total + kSmallBflies - 1) / kSmallBflies),
                      (unsigned)(8 * kSmallBflies), s, out, (int)T.N, B, n, nodes, (int)T.level_count[lv],
-                     (const uint32_t *)T.tw, (const uint8_t *)T.dneg, (int)T.tws);
-    else if (L <= kPackedTwiddleMaxLimbs && B % lthreads == 0)
-      mp_level_kernel<L, (L <= kPackedTwiddleMaxLimbs)><<<blocks, lthreads, 0, s>>>(
-          out, T.N, B, n, T.node_off + T.level_start[lv], T.level_count[lv], T.tw, T.dneg, T.tws);
+                     (const uint32_t *)T.twp, (const uint8_t *)T.dneg, (int)T.tws);
     else
-      mp_level_kernel<L, false><<<blocks, lthreads, 0, s>>>(out, T.N, B, n, T.node_off + T.level_start[lv],
-                                                            T.level_count[lv], T.tw, T.dneg, T.tws);
+      mp_level_kernel<L><<<blocks, lthreads, 0, s>>>(out, T.N, B, n, T.node_off + T.level_start[lv],
+                                                     T.level_count[lv], T.twp, T.dneg, T.tws);
     if (e != cudaSuccess) return e;
     timer.end();
   }

@@ -161,7 +161,7 @@ __device__ __forceinline__ void combine_p(uint32_t (&x)[L], const uint32_t *p, s
 // so that costs (N=1024, batch 2048, us per batch, that form / this one): 9
 // limbs 470 / 432, 17 limbs 1057 / 907, 25 limbs 1810 / 1521, 33 limbs 2810 / 2330.
 //
-// kPacked: w holds the L limbs contiguously in shared memory, 16-byte aligned
+// kPacked: w holds the L limbs contiguously, 16-byte aligned
 // (tplane unused); they are read four at a time with 128-bit loads.
 template <int L, bool kPacked = false>
 __device__ __forceinline__ void mul_tw(uint32_t (&x)[L], const uint32_t *w, size_t tplane) {

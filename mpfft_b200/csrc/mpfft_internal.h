@@ -251,7 +251,7 @@ cudaError_t d_real_split(bool forward, const double *in, double *out, int M, int
 struct QueueTables {
   int N = 0;
   TreeTables tree;                 // limb forms
-  const uint32_t *tw = nullptr;    // limb forms: [3][L][N/4]
+  const uint32_t *twp = nullptr;   // limb forms: the packed twiddles (MpDeviceTables)
   const uint8_t *dneg = nullptr;
   DDeviceTables ft;                // floating forms
 };

@@ -56,8 +56,7 @@ __global__ void __launch_bounds__(256) mp_queue_kernel(const QueueItem *__restri
       const int total = T.level_count[lv] * q;
       const int *nodes = T.node_off + T.level_start[lv];
       for (int t = threadIdx.x; t < total; t += blockDim.x)
-        mp_bfly_one<L, false>(out, N, 1, 0, n, nodes[t / q], t % q, Q.tw, Q.dneg, 1, Ps + threadIdx.x, blockDim.x,
-                              nullptr);
+        mp_bfly_one<L>(out, N, 1, 0, n, nodes[t / q], t % q, Q.twp, Q.dneg, 1, Ps + threadIdx.x, blockDim.x);
     }
   }
 }
