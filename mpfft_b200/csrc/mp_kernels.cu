@@ -270,12 +270,136 @@ constexpr int pair_min_blocks() {
   return L >= 31 ? 3 : level_min_blocks<L>();
 }
 
+// one word of global memory to shared memory, asynchronously
+__device__ __forceinline__ void cp_async_word(uint32_t *dst, const uint32_t *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void prefetch_l2(const uint32_t *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
+
+constexpr int kPairThreads = 128;
+
+// Whether the pair kernel's threads fetch a side's Z slot into shared memory
+// while the side before it is multiplied (mp_pair_steps), or read it where a
+// step needs it (mp_bfly_steps).  With three CTAs per SM a warp that waits for
+// its loads is rarely covered by the other two of its scheduler; from 31 limbs
+// that outweighs the copies (N=1024, batch 2048, us per batch, read / fetched:
+// 9 limbs 436 / 452, 17 limbs 906 / 911, 25 limbs 1462 / 1444, 33 limbs 2285 / 2211;
+// 65536 points, batch 24, 34 limbs 3500 / 3404).
 template <int L>
-__global__ void __launch_bounds__(128, pair_min_blocks<L>()) mp_level_pair_kernel(
+constexpr bool pair_async = L >= 31;
+template <int L>
+constexpr int pair_smem = (pair_async<L> ? 3 : 1) * L * kPairThreads * 4;
+
+// The twiddle steps of a thread of mp_level_pair_kernel (the table above): of
+// X's butterfly k, then (fused) Y's butterflies k and k+q; p: position k of the
+// node.  S: this thread's column of 3L words of shared memory (stride
+// kPairThreads): the side's first product P, and the real and imaginary words
+// of the side's Z slot.  A word of the next side takes the place of this side's
+// as soon as the step that reads it last has it in registers, so each has one or
+// two products' time to arrive; each thread waits for its own copies only.
+template <int L>
+__device__ __forceinline__ void mp_pair_steps(uint32_t *p, size_t qB, size_t plane, size_t cim, int N, int n, int k,
+                                              bool fused, const uint32_t *__restrict__ twp,
+                                              const uint8_t *__restrict__ dneg, int tws, uint32_t *S) {
+  constexpr int Lp = (L + 3) & ~3;  // packed twiddle stride: 16-byte aligned rows
+  constexpr size_t ps = kPairThreads;
+  uint32_t *Sr = S + (size_t)L * ps, *Si = S + (size_t)2 * L * ps;
+  const int q = n >> 2;
+  const int end = fused ? 6 : 2;
+  const int first = k ? 0 : 4;  // (butterfly k = 0 of X and of Y: no twiddle)
+  if (first >= end) return;
+  // side s: Z+ / Z- of X at 2q, 3q, of Y_k at 4q, 6q, of Y_{k+q} at 5q, 7q
+  auto slot = [&](int s) { return p + (size_t)(s < 2 ? 2 + s : 3 + (s >> 1) + 2 * (s & 1)) * qB; };
+  auto fetch = [&](uint32_t *dst, const uint32_t *src) {
+#pragma unroll
+    for (int i = 0; i < L; ++i) cp_async_word(dst + (size_t)i * ps, src + (size_t)i * plane);
+  };
+  fetch(Sr, slot(first));
+  fetch(Si, slot(first) + cim);
+  uint32_t X[L];
+  int side = first, step = 0;
+#pragma unroll 1
+  for (; side < end;) {
+    const int j = side >> 1;
+    const bool minus = side & 1;
+    const int kk = j == 2 ? k + q : k, nn = j == 0 ? n : 2 * n;
+    const int kn = kk * (N / nn) * tws;
+    const bool special = 8 * kk == nn;
+    const bool dn = special ? false : (dneg[kn] != 0);
+    uint32_t *zr = slot(side);
+    const uint32_t *pa = Sr, *pb = nullptr;
+    int wsel = 0;  // packed twiddle row: 0 cos, 1 cos+sin, 2 |cos-sin|
+    bool sub = false, negx = false, mul = true;
+    int sp = 0;
+    uint32_t *dst = nullptr;  // null: the product becomes P
+    bool next_r = false, next_i = false;  // the side's word that was read for the last time
+    if (step == 0) {
+      cp_async_wait();
+      pb = Si;
+      sub = minus;
+    } else if (!special) {
+      if (step == 1) {
+        pa = Si;
+        wsel = 2;
+        negx = dn ^ !minus;
+        sp = 1;
+        dst = zr + cim;
+        next_i = true;
+      } else {
+        wsel = 1;
+        negx = !minus;
+        sp = minus ? -1 : 1;
+        dst = zr;
+        next_r = true;
+      }
+    } else {
+      if (step == 1) {
+        pa = minus ? Sr : Si;
+        pb = minus ? Si : Sr;
+        sub = !minus;
+        dst = zr;
+        next_r = next_i = true;
+      } else {
+        mul = false;
+        sp = 1;
+        dst = zr + cim;
+      }
+    }
+    if (mul) {
+      ld_addsub<L>(X, pa, pb, ps, sub);
+      if (side + 1 < end) {
+        if (next_r) fetch(Sr, slot(side + 1));
+        if (next_i) fetch(Si, slot(side + 1) + cim);
+      }
+      else if (step == 0) {  // the U slots (at 0 and q), read by the combine
+        for (int e = threadIdx.x & 31; e < 4 * L; e += 32)
+          prefetch_l2(p + (e >= 2 * L ? qB : 0) + (size_t)(e >= 2 * L ? e - 2 * L : e) * plane);
+      }
+      mul_tw<L, true>(X, twp + (size_t)kn * (3 * Lp) + wsel * Lp, 0);
+    } else {
+#pragma unroll
+      for (int i = 0; i < L; ++i) X[i] = 0;
+    }
+    if (!dst) {
+      st<L>(S, ps, X);
+    } else {
+      combine_p<L>(X, S, ps, negx, sp);
+      const uint64_t keep = l2_policy_evict_last();
+#pragma unroll
+      for (int i = 0; i < L; ++i) st_hint(dst + (size_t)i * plane, X[i], keep);
+    }
+    if (++step == 3) step = 0, ++side;
+  }
+}
+
+template <int L>
+__global__ void __launch_bounds__(kPairThreads, pair_min_blocks<L>()) mp_level_pair_kernel(
     uint32_t *__restrict__ y, int N, int B, int n, const int *__restrict__ ynodes, int ny,
     const int *__restrict__ unodes, int nu, const uint32_t *__restrict__ twp, const uint8_t *__restrict__ dneg,
     int tws) {
-  __shared__ uint32_t Ps[L * 128];
+  extern __shared__ uint32_t pair_words[];
   const int q = n >> 2;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nf = (long long)ny * q * B;
@@ -292,13 +416,17 @@ __global__ void __launch_bounds__(128, pair_min_blocks<L>()) mp_level_pair_kerne
   uint32_t *p = y + (size_t)(off + k) * B + b;
   // the twiddle steps: X's (or the unfused node's) butterfly k, then Y's
   // butterflies k and k+q; one inlined copy of the product
+  if constexpr (pair_async<L>) {
+    mp_pair_steps<L>(p, qB, plane, cim, N, n, k, fused, twp, dneg, tws, pair_words + threadIdx.x);
+  } else {
 #pragma unroll 1
-  for (int j = 0; j < (fused ? 3 : 1); ++j) {
-    const int kk = j == 2 ? k + q : k;
-    if (kk == 0) continue;
-    const int zs = j == 0 ? 2 : (j == 1 ? 4 : 5);  // Z+ slot at zs*q, Z- at (zs+1)*q or (zs+2)*q
-    mp_bfly_steps<L>(p + (size_t)zs * qB, p + (size_t)(j == 0 ? 3 : zs + 2) * qB, plane, cim, N, j == 0 ? n : 2 * n, kk,
-                     twp, dneg, tws, Ps + threadIdx.x, blockDim.x);
+    for (int j = 0; j < (fused ? 3 : 1); ++j) {
+      const int kk = j == 2 ? k + q : k;
+      if (kk == 0) continue;
+      const int zs = j == 0 ? 2 : (j == 1 ? 4 : 5);  // Z+ slot at zs*q, Z- at (zs+1)*q or (zs+2)*q
+      mp_bfly_steps<L>(p + (size_t)zs * qB, p + (size_t)(j == 0 ? 3 : zs + 2) * qB, plane, cim, N,
+                       j == 0 ? n : 2 * n, kk, twp, dneg, tws, pair_words + threadIdx.x, kPairThreads);
+    }
   }
   if (fused) combine_pair<L>(p, qB, plane, cim, k != 0);
   else combine<L>(p, p + qB, p + 2 * qB, p + 3 * qB, plane, cim, k != 0);
@@ -686,8 +814,14 @@ static cudaError_t run_transform(const MpDeviceTables &T, const uint32_t *in, ui
         (long long)T.level_count[lv + 1] * (n / 2) * B >= kSmallLevelButterflies) {
       // levels lv and lv+1 in one launch; lv+1's timer entry stays 0
       const long long threads = fused + (long long)T.pair_count[lv] * (n / 4) * B;
+      constexpr int smem = pair_smem<L>;
+      if (smem > 49152) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(mp_level_pair_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+      }
       timer.begin();
-      mp_level_pair_kernel<L><<<(unsigned)((threads + lthreads - 1) / lthreads), lthreads, 0, s>>>(
+      mp_level_pair_kernel<L><<<(unsigned)((threads + kPairThreads - 1) / kPairThreads), kPairThreads, smem, s>>>(
           out, T.N, B, n, T.node_off + T.level_start[lv + 1], T.level_count[lv + 1],
           T.pair_nodes + T.pair_start[lv], T.pair_count[lv], T.twp, T.dneg, T.tws);
       timer.end();

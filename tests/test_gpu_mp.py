@@ -426,3 +426,31 @@ def test_mp_tiles_bit_identical(M, n, p, B):
         ref = torch.empty_like(one)
         plan.execute_device_timed(1, one.data_ptr(), ref.data_ptr(), s)
         assert torch.equal(d_out[..., b].contiguous(), ref), b
+
+
+@pytest.mark.parametrize("n,limbs,B", [(16, 30, 16001), (16, 31, 10501), (32, 31, 5003), (32, 34, 5024), (64, 32, 2611),
+                                       (128, 33, 1301), (256, 34, 641)])
+def test_mp_pairs_past_the_tiles_bit_identical(M, n, limbs, B):
+    """Batches past the tiles' range: two levels per launch, the Z slots read in
+    place (30 limbs) or fetched ahead through shared memory (from 31), with and
+    without a level left over, batches that cut warps.  Signals cut from the
+    batch run alone, one level per launch: the outputs are bit-identical."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    plan = M.MpPlan(n, 32 * limbs - 7 - 2 * (n.bit_length() - 1))
+    L = plan.limbs
+    assert L == limbs
+    host = synthetic_planes(n, L, plan.frac_bits, 61, seed=n + B).reshape(2, L, n, 61)
+    s = torch.cuda.current_stream().cuda_stream
+    some = torch.from_numpy(np.ascontiguousarray(host).view(np.int32)).cuda()
+    d_in = some[..., torch.arange(B, device="cuda") % 61].contiguous()
+    d_out = torch.full_like(d_in, -1)
+    plan.execute_device(B, d_in.data_ptr(), d_out.data_ptr(), s)
+    ref = torch.empty_like(some)
+    for b in range(61):
+        one, out = some[..., b].contiguous(), torch.empty_like(some[..., b]).contiguous()
+        plan.execute_device_timed(1, one.data_ptr(), out.data_ptr(), s)
+        ref[..., b] = out
+    assert torch.equal(d_out, ref[..., torch.arange(B, device="cuda") % 61])
