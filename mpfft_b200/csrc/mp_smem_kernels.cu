@@ -46,13 +46,24 @@ template <int L>
 __host__ __device__ constexpr int smem_lg_tile() {
   return L <= 18 ? 9 : 8;
 }
-template <int L>
+// Threads of a CTA: P/4, or P/2 (WIDE), which takes a level's butterflies in one
+// round where the other takes two, but leaves room for fewer CTAs: their
+// registers, not shared memory, then limit them.  smem_min_blocks: CTAs per SM.
+template <int L, bool WIDE>
 __host__ __device__ constexpr int tile_threads() {
-  return 1 << (smem_lg_tile<L>() - 2);
+  return 1 << (smem_lg_tile<L>() - (WIDE ? 1 : 2));
 }
-template <int L>
+template <int L, bool WIDE>
 __host__ __device__ constexpr int smem_min_blocks() {
-  return L <= 4 ? 8 : L <= 6 ? 6 : L <= 10 ? 5 : L <= 14 ? 4 : L <= 18 ? 3 : L <= 21 ? 5 : L <= 27 ? 4 : 3;
+  return WIDE ? (L <= 18 ? 2 : L <= 21 ? 4 : L <= 27 ? 3 : 2)
+              : (L <= 4 ? 8 : L <= 6 ? 6 : L <= 10 ? 5 : L <= 14 ? 4 : L <= 18 ? 3 : L <= 27 ? 4 : 3);
+}
+// Limb counts whose tiles are always wide: four wide CTAs per SM without spills
+// (20 limbs, us, narrow / wide: 65 k points 100 / 83, 131 k 101 / 94, 410 k
+// 379 / 330, 524 k 355 / 343, 2 M 1267 / 1259)
+template <int L>
+__host__ __device__ constexpr bool tile_always_wide() {
+  return L >= 19 && L <= 21;
 }
 
 struct MpTile {
@@ -343,8 +354,8 @@ __device__ __forceinline__ void tile_level(const MpTile &A, uint32_t *sm, const 
   }
 }
 
-template <int L, bool LEAF>
-__global__ void __launch_bounds__(tile_threads<L>(), smem_min_blocks<L>())
+template <int L, bool LEAF, bool WIDE>
+__global__ void __launch_bounds__(tile_threads<L, WIDE>(), smem_min_blocks<L, WIDE>())
     mp_tile_kernel(const __grid_constant__ MpTile A) {
   extern __shared__ __align__(16) uint32_t tile_smem[];
   constexpr int P = 1 << smem_lg_tile<L>();
@@ -430,16 +441,34 @@ cudaError_t mp_pack_tw(const uint32_t *tw, uint32_t *twp, int L, long long n4, c
   return cudaGetLastError();
 }
 
-template <int L, bool LEAF>
-static cudaError_t tile_launch(const MpTile &A, cudaStream_t s) {
+template <int L, bool LEAF, bool WIDE>
+static cudaError_t tile_launch(const MpTile &A, long long ctas, cudaStream_t s) {
   constexpr int P = 1 << smem_lg_tile<L>();
   const size_t smem = (size_t)8 * L * P + ((size_t)(LEAF ? 10 : 2) << (A.lgM - 2)) + 8;
-  const cudaError_t e = cudaFuncSetAttribute(mp_tile_kernel<L, LEAF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             8 * L * P + 10 * P / 4 + 8);
+  const cudaError_t e = cudaFuncSetAttribute(mp_tile_kernel<L, LEAF, WIDE>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * L * P + 10 * P / 4 + 8);
   if (e != cudaSuccess) return e;
-  const long long ctas = ((long long)A.N >> (A.lgM + A.lgu)) * A.groups;
-  mp_tile_kernel<L, LEAF><<<(unsigned)ctas, tile_threads<L>(), smem, s>>>(A);
+  mp_tile_kernel<L, LEAF, WIDE><<<(unsigned)ctas, tile_threads<L, WIDE>(), smem, s>>>(A);
   return cudaGetLastError();
+}
+
+// Launches whose tiles all run at once as wide CTAs take those, to 14 limbs
+// only while no SM gets two (us, narrow / wide: 4 limbs 16 k points 22.2 / 19.9;
+// 9 limbs 66 k 40.7 / 37.4; 17 limbs 33 k 68.6 / 55.8, 131 k 83.3 / 75.5; 23 limbs 66 k
+// 115.8 / 94.8; 33 limbs 66 k 184 / 149).  Past that the narrow ones, of which more
+// fit, are the faster or the same (11 limbs 131 k 48.9 / 50.1, 205 k 58.3 / 63.2;
+// 9 limbs 2 M 329 / 409; 17 limbs 410 k 267 / 284; 25 limbs 131 k 130 / 153; 33 limbs
+// 524 k 849 / 901).
+template <int L>
+constexpr int kWideTilesPerSm = L <= 14 ? 1 : smem_min_blocks<L, true>();
+
+template <int L, bool LEAF>
+static cudaError_t tile_launch(const MpTile &A, cudaStream_t s) {
+  const long long ctas = ((long long)A.N >> (A.lgM + A.lgu)) * A.groups;
+  if constexpr (!tile_always_wide<L>()) {
+    if (ctas > 148LL * kWideTilesPerSm<L>) return tile_launch<L, LEAF, false>(A, ctas, s);
+  }
+  return tile_launch<L, LEAF, true>(A, ctas, s);
 }
 
 static int lg2(long long n) { return 63 - __builtin_clzll((unsigned long long)n); }
@@ -480,25 +509,29 @@ static cudaError_t tile_run(const MpDeviceTables &T, const uint32_t *in, uint32_
   return e;
 }
 
-// Which transforms run in tiles (points N*B by limb count), measured over N =
-// 32 .. 16384, B = 1 .. 4096 against one launch per level or level pair:
-//   from   a tile's latency (about 10 + 4L us a launch) is hidden by the others
-//          (9 limbs: 8 k points 0.97x, 16 k 1.25x, 37 k 1.4x, 131 k 2.2x; 17 limbs
-//          32 k 0.99x, 65 k 1.36x, 131 k 1.8x; 33 limbs 32 k 0.85x, 65 k 1.4x)
+// Which transforms run in tiles (points N*B by limb count), measured over N = 64
+// .. 16384, B = 1 .. 1536 against one launch per level or level pair:
+//   from   a tile's latency is hidden by the others; long single signals, which
+//          take a launch more, last (4 limbs: 4 k points 1.00x, 8 k 1.01 .. 1.15x;
+//          9 limbs: 8 k 0.88 .. 1.06x, 16 k 1.12 .. 1.27x; 12 limbs: 16 k 0.92 ..
+//          1.09x, 20 k 1.16x; 17 limbs 25 k 0.85 .. 1.01x, 33 k 1.05 .. 1.18x; 33
+//          limbs 25 k 0.88 .. 0.98x, 33 k 1.08 .. 1.41x)
 //   to     large batches fill the GPU level by level too, and from 15 limbs up
 //          the register-resident kernels keep more products in flight than a
-//          tile's share of shared memory does (13 limbs 4 M points 1.09x; 17 limbs
-//          1 M 1.07x, 4 M 0.95x; 25 limbs 524 k 1.15x, 1 M 0.86x; 33 limbs 131 k
-//          1.25x, 262 k 0.89x)
+//          tile's share of shared memory does (12 limbs 1.5 M points 1.11x, 14 limbs
+//          1.5 M 0.99x; 17 limbs 1 M 1.04x, 1.5 M 0.93x; 20 limbs 786 k 1.08x, 1 M
+//          0.90x; 25 limbs 262 k 1.16x, 328 k 0.94x; 30 limbs 205 k 1.16x, 262 k 0.96x;
+//          33 limbs 131 k 1.23x, 164 k 0.98x, 262 k 0.84x)
 bool mp_tile_used(const MpDeviceTables &T, int L, int B) {
   if (!T.twp || L > kMaxLimbs || T.N < 16) return false;
   const long long w = (long long)T.N * B;
-  const long long from = L <= 7 ? 8192 : L <= 9 ? 12288 : L <= 11 ? 24576 : L <= 13 ? 32768 : 49152;
+  const long long from = L <= 6 ? 8192 : L <= 9 ? 12288 : L <= 12 ? 20000 : 28672;
   const long long to = L <= 14   ? (1LL << 62)
-                       : L <= 20 ? 1500000
-                       : L <= 27 ? 700000
+                       : L <= 18 ? 1200000
+                       : L <= 21 ? 900000
+                       : L <= 27 ? 300000
                        : L <= 30 ? 250000
-                                 : 160000;
+                                 : 150000;
   return w >= from && w <= to;
 }
 

@@ -454,3 +454,29 @@ def test_mp_pairs_past_the_tiles_bit_identical(M, n, limbs, B):
         plan.execute_device_timed(1, one.data_ptr(), out.data_ptr(), s)
         ref[..., b] = out
     assert torch.equal(d_out, ref[..., torch.arange(B, device="cuda") % 61])
+
+
+@pytest.mark.parametrize("n,p,B", [(1024, 100, 74), (1024, 256, 74), (1024, 256, 75), (512, 380, 147), (1024, 500, 148),
+                                   (1024, 500, 149), (4096, 580, 7), (256, 600, 301), (1024, 760, 111),
+                                   (1024, 760, 112), (1024, 1020, 74), (1024, 1020, 75), (32768, 1000, 1)])
+def test_mp_wide_tiles_bit_identical(M, n, p, B):
+    """Tile launches up to and past the tiles that run at once with twice the
+    threads (148 of 512 points to 14 limbs, 296 to 18, 444 and 296 of 256 points at
+    25 and 33), and limb counts that always take them.  Single signals cut from
+    the batch run level by level: the outputs are bit-identical."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    plan = M.MpPlan(n, p)
+    L = plan.limbs
+    host = synthetic_planes(n, L, plan.frac_bits, B, seed=n + B).reshape(2, L, n, B)
+    s = torch.cuda.current_stream().cuda_stream
+    d_in = torch.from_numpy(np.ascontiguousarray(host).view(np.int32)).cuda()
+    d_out = torch.full_like(d_in, -1)
+    plan.execute_device(B, d_in.data_ptr(), d_out.data_ptr(), s)
+    for b in range(0, B, 7 if B > 7 else 1):
+        one = d_in[..., b].contiguous()
+        ref = torch.empty_like(one)
+        plan.execute_device_timed(1, one.data_ptr(), ref.data_ptr(), s)
+        assert torch.equal(d_out[..., b].contiguous(), ref), b
