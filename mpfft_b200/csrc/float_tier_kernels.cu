@@ -13,9 +13,14 @@ namespace mpfft {
 // 160; quad-double with one level per pass 582, with 192 threads 631, three CTAs
 // of 192 (spilling) 686, two levels per pass (8 points, 255 registers) 896.  One
 // CTA of 512 threads with a chunk twice as large, which saves a pass above:
-// double-double 152, quad-double 617.
-template <class NT, bool SINGLE>
-__global__ void __launch_bounds__(256, 2)
+// double-double 152, quad-double 617.  FEW (fewer chunks than SMs, one each of at
+// most 2^kLgFew points): a CTA has its SM to itself and takes all the registers
+// (quad-double, one signal, us, two CTAs' registers / all: 16 points 11.2 / 8.8,
+// 128 points 21.9 / 16.4, 1024 points 42.4 / 37.7; double-double with base cases of
+// eight / four positions: 16 points 4.6 / 4.3, 128 points 7.5 / 7.0, but 2048 points
+// 22.6 / 24.2).
+template <class NT, bool SINGLE, bool FEW>
+__global__ void __launch_bounds__(256, FEW ? 1 : 2)
     tier_sub_kernel(const __grid_constant__ TierTab S, TierArgs<NT> A, int groups) {
   extern __shared__ __align__(16) double2 tier_smem[];
   const int g = A.G;
@@ -27,7 +32,7 @@ __global__ void __launch_bounds__(256, 2)
     A.c0 = (blockIdx.x % groups) * g;
     A.G = min(g, S.nchunks - A.c0);
   }
-  tier_sub_transform<NT, SINGLE>(S, A, tier_smem);
+  tier_sub_transform<NT, SINGLE, FEW>(S, A, tier_smem);
 }
 
 template <class NT>
@@ -65,27 +70,33 @@ cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaSt
   return cudaGetLastError();
 }
 
+template <class NT, bool SINGLE, bool FEW>
+static cudaError_t tier_sub_launch(const TierTab &S, TierArgs<NT> A, cudaStream_t s) {
+  const size_t smem = ((size_t)A.G << S.lgT) * NT::kUnits * sizeof(double2) + kOrderBytes;
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(tier_sub_kernel<NT, SINGLE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (NT::kUnits << NT::kLgMax) * (int)sizeof(double2) + (int)kOrderBytes);
+    if (e != cudaSuccess) return e;
+  }
+  const int threads = std::min(256, std::max(32, (A.G << S.lgT) >> (A.per + 1)));
+  const int groups = SINGLE ? 1 : (S.nchunks + A.G - 1) / A.G;
+  const long long ctas = SINGLE ? ((long long)A.B + A.G - 1) / A.G : (long long)groups * A.B;
+  tier_sub_kernel<NT, SINGLE, FEW><<<(unsigned)ctas, threads, smem, s>>>(S, A, groups);
+  return cudaGetLastError();
+}
+
 template <class NT, bool SINGLE>
 static cudaError_t tier_sub_launch(const TierTab &S, TierArgs<NT> A, cudaStream_t s) {
   // chunks per CTA: as many as fit, but no more than leave two CTAs for every SM
   const long long inst = SINGLE ? A.B : (long long)S.nchunks * A.B;
-  int g = 1 << (NT::kLgMax - S.lgT);
-  while (g > 1 && inst / g < 2 * 148) g /= 2;
-  A.G = g;
+  A.G = 1 << (NT::kLgMax - S.lgT);
+  while (A.G > 1 && inst / A.G < 2 * 148) A.G /= 2;
   // few CTAs: one level per pass, so that each pass has the most threads (one
   // 1024-point float-float signal: 14.4 us with three levels per pass)
-  A.per = inst / g < 148 ? 1 : NT::kLevels;
-  const size_t smem = ((size_t)g << S.lgT) * NT::kUnits * sizeof(double2) + kOrderBytes;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(tier_sub_kernel<NT, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (NT::kUnits << NT::kLgMax) * (int)sizeof(double2) + (int)kOrderBytes);
-    if (e != cudaSuccess) return e;
-  }
-  const int threads = std::min(256, std::max(32, (g << S.lgT) >> (A.per + 1)));
-  const int groups = SINGLE ? 1 : (S.nchunks + g - 1) / g;
-  const long long ctas = SINGLE ? ((long long)A.B + g - 1) / g : (long long)groups * A.B;
-  tier_sub_kernel<NT, SINGLE><<<(unsigned)ctas, threads, smem, s>>>(S, A, groups);
-  return cudaGetLastError();
+  A.per = inst / A.G < 148 ? 1 : NT::kLevels;
+  if (inst < 148 && S.lgT <= NT::kLgFew) return tier_sub_launch<NT, SINGLE, true>(S, A, s);
+  return tier_sub_launch<NT, SINGLE, false>(S, A, s);
 }
 
 template <class NT>
@@ -127,7 +138,8 @@ int tier_sub_max(int tier) {
 int tier_tw_words(int tier) {
   return tier == kTierQD ? QDT::kTwWords : tier == kTierFF ? FFT_::kTwWords : DDT::kTwWords;
 }
-int tier_leaf_lg(int tier) {
+int tier_leaf_lg(int tier, bool few) {
+  if (few) return tier == kTierQD ? QDT::kLeafLgFew : tier == kTierFF ? FFT_::kLeafLgFew : DDT::kLeafLgFew;
   return tier == kTierQD ? QDT::kLeafLg : tier == kTierFF ? FFT_::kLeafLg : DDT::kLeafLg;
 }
 int tier_pass_levels(int tier) {

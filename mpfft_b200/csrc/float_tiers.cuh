@@ -92,6 +92,7 @@ struct DDT {
   static constexpr int K = 2;
   static constexpr int kLgMax = 11;   // lg of the largest chunk (64 KB)
   static constexpr int kLeafLg = 3;   // lg of the positions of a base-case slot
+  static constexpr int kLeafLgFew = 2, kLgFew = 9;  // the same for one chunk alone, up to 2^kLgFew points
   static constexpr int kLevels = 2;   // levels per pass
 
   // accurate addition (two TwoSums, two renormalisations)
@@ -169,6 +170,7 @@ struct QDT {
   static constexpr int K = 4;
   static constexpr int kLgMax = 10;
   static constexpr int kLeafLg = 2;
+  static constexpr int kLeafLgFew = 2, kLgFew = 10;
   static constexpr int kLevels = 1;
 
   // Sum order by order: word i of x and of y are order i; the error of an
@@ -247,6 +249,7 @@ struct FFT_ {
   static constexpr int K = 2;
   static constexpr int kLgMax = 12;
   static constexpr int kLeafLg = 3;
+  static constexpr int kLeafLgFew = 3, kLgFew = 9;
   static constexpr int kLevels = 3;
 
   static __device__ __forceinline__ V add(V a, V b) {
@@ -384,6 +387,10 @@ __device__ __forceinline__ void tier_levels(Pt<NT> (&v)[2 << R], bool big, const
   typename NT::TW c, s;
   if constexpr (R == 1) {
     if (!big) return;
+    if (NT::kLeafLg == 3 && u == 2 && k == 0) {  // as in the 8-position base case: the same bits
+      leaf8_k0<NT>(v[0], v[1], v[2], v[3]);
+      return;
+    }
     tier_tw<NT>(S, 4 * u, k, c, s);
     bfly<NT>(v[0], v[1], v[2], v[3], c, s);
   } else if constexpr (R == 2) {
@@ -443,16 +450,17 @@ struct TierArgs {
 // positions; either way the slot's inputs are of one class mod N/2^kLeafLg:
 //   8  a node of 8 points (a leaf of 4, two of 2, and the level above) or two leaves of 4
 //   4  a leaf of 4 or two of 2 (quad-double: eight points do not fit in registers)
-template <class NT, bool SINGLE>
+template <class NT, bool SINGLE, bool FEW>
 __device__ __forceinline__ void tier_leaves(const TierTab &S, const TierArgs<NT> &A, double2 *sm) {
-  constexpr int kLg = NT::kLeafLg, kPts = 1 << kLg;
-  const int lgT = S.lgT, nslots = 1 << (lgT - kLg), pl = A.G << lgT, N = S.N;
+  constexpr int kLg = FEW ? NT::kLeafLgFew : NT::kLeafLg, kPts = 1 << kLg;
+  const int G = FEW ? 1 : A.G;
+  const int lgT = S.lgT, nslots = 1 << (lgT - kLg), pl = G << lgT, N = S.N;
   const size_t hplane = (size_t)A.B * N, cplane = (size_t)NT::K * hplane;
   const size_t in_re = A.swap_in ? cplane : 0, in_im = A.swap_in ? 0 : cplane;
-  for (int e = threadIdx.x; e < A.G * nslots; e += blockDim.x) {
-    const int g = SINGLE ? e / nslots : e % A.G;
-    int s = SINGLE ? e % nslots : e / A.G;
-    int half = 0, sna = 0, rs = 1, chunk = 0;
+  for (int e = threadIdx.x; e < G * nslots; e += blockDim.x) {
+    const int g = FEW ? 0 : SINGLE ? e / nslots : e % G;
+    int s = FEW ? e : SINGLE ? e % nslots : e / G;
+    int half = 0, sna = 0, rs = 1, chunk = 0, lgt = lgT;
     const TierLeafSlot *tab = S.slots[0];
     if (!SINGLE) {
       const SrChunk ch = S.chunks[A.c0 + g];
@@ -461,12 +469,14 @@ __device__ __forceinline__ void tier_leaves(const TierTab &S, const TierArgs<NT>
       rs = N >> lgT;
       if (!sr_chunk_big(chunk)) {
         tab = S.slots[1];
+        --lgt;
         rs *= 2;
         half = s >= nslots / 2;
         s -= half ? nslots / 2 : 0;
         if (half) sna = ch.snb;
       }
     }
+    if (kLg != NT::kLeafLg) tab += 1 << (lgt - NT::kLeafLg);  // behind the slots of 2^kLeafLg positions
     const TierLeafSlot L = tab[s];
     const int m = half * (nslots / 2) + L.m;
     const bool big = sr_chunk_big(chunk * nslots + m);
@@ -536,10 +546,11 @@ __device__ __forceinline__ void tier_fill_order(uint16_t *order, int chunks) {
 }
 
 // R levels of every chunk of 2^(R+1)*u positions, u = 2^lgu; last: to global memory
-template <class NT, int R, bool SINGLE>
+template <class NT, int R, bool SINGLE, bool FEW>
 __device__ __forceinline__ void tier_pass(const TierTab &S, const TierArgs<NT> &A, double2 *sm, int lgu, bool last) {
   constexpr int M = 2 << R;
-  const int lgT = S.lgT, pl = A.G << lgT, u = 1 << lgu, lgc = lgu + R + 1, lgnch = lgT - lgc;
+  const int G = FEW ? 1 : A.G;
+  const int lgT = S.lgT, pl = G << lgT, u = 1 << lgu, lgc = lgu + R + 1, lgnch = lgT - lgc;
   const size_t hplane = (size_t)A.B * S.N, cplane = (size_t)NT::K * hplane;
   int off[M];
 #pragma unroll
@@ -549,8 +560,8 @@ __device__ __forceinline__ void tier_pass(const TierTab &S, const TierArgs<NT> &
   // one level alone only has work in the nodes (and in a pair's last chunk, see above)
   const bool only = R == 1 && !last;
   const int slots = only ? nodes + (!SINGLE && (lgnch & 1) ? 1 : 0) : nch;
-  for (int e = threadIdx.x; e < (A.G * slots) << lgu; e += blockDim.x) {
-    const int k = e & (u - 1), x = e >> lgu, g = only ? x / slots : x >> lgnch, i = x - g * slots;
+  for (int e = threadIdx.x; e < (G * slots) << lgu; e += blockDim.x) {
+    const int k = e & (u - 1), x = e >> lgu, g = FEW ? 0 : only ? x / slots : x >> lgnch, i = x - g * slots;
     const int ci = i < nodes ? order[i] : only ? nch - 1 : order[kOrderPairs + i - nodes], c = (g << lgnch) + ci;
     const int chunk = SINGLE ? 0 : __ldg(&S.chunks[A.c0 + g].chunk);
     const bool big = sr_chunk_big((chunk << lgnch) + ci);
@@ -573,12 +584,15 @@ __device__ __forceinline__ void tier_pass(const TierTab &S, const TierArgs<NT> &
   }
 }
 
-// T = 2^lgT >= 8
-template <class NT, bool SINGLE>
+// T = 2^lgT >= 8.  FEW: one chunk (A.G = 1) of few points: one level per pass
+// (A.per = 1) and base cases of 2^kLeafLgFew positions, so that the most threads
+// have work and none has much.
+template <class NT, bool SINGLE, bool FEW>
 __device__ __forceinline__ void tier_sub_transform(const TierTab &S, const TierArgs<NT> &A, double2 *sm) {
-  tier_fill_order(tier_order(sm, (A.G << S.lgT) * NT::kUnits), 1 << (S.lgT - NT::kLeafLg) >> 1);
-  tier_leaves<NT, SINGLE>(S, A, sm);
-  int done = NT::kLeafLg;
+  constexpr int kLg = FEW ? NT::kLeafLgFew : NT::kLeafLg;
+  tier_fill_order(tier_order(sm, (A.G << S.lgT) * NT::kUnits), 1 << (S.lgT - kLg) >> 1);
+  tier_leaves<NT, SINGLE, FEW>(S, A, sm);
+  int done = kLg;
   if (done == S.lgT) {  // (8 points) the base cases are the transform
     __syncthreads();
     const size_t hplane = (size_t)A.B * S.N, cplane = (size_t)NT::K * hplane;
@@ -591,12 +605,13 @@ __device__ __forceinline__ void tier_sub_transform(const TierTab &S, const TierA
     return;
   }
   while (done < S.lgT) {
-    const int r = min(A.per, S.lgT - done);
+    const int r = FEW ? 1 : min(A.per, S.lgT - done);
     const bool last = done + r == S.lgT;
     __syncthreads();
-    if (NT::kLevels == 3 && r == 3) tier_pass<NT, NT::kLevels, SINGLE>(S, A, sm, done - 1, last);
-    else if (NT::kLevels >= 2 && r == 2) tier_pass<NT, NT::kLevels >= 2 ? 2 : 1, SINGLE>(S, A, sm, done - 1, last);
-    else tier_pass<NT, 1, SINGLE>(S, A, sm, done - 1, last);
+    if (FEW) tier_pass<NT, 1, SINGLE, true>(S, A, sm, done - 1, last);
+    else if (NT::kLevels == 3 && r == 3) tier_pass<NT, NT::kLevels, SINGLE, false>(S, A, sm, done - 1, last);
+    else if (NT::kLevels >= 2 && r == 2) tier_pass<NT, NT::kLevels >= 2 ? 2 : 1, SINGLE, false>(S, A, sm, done - 1, last);
+    else tier_pass<NT, 1, SINGLE, false>(S, A, sm, done - 1, last);
     done += r;
   }
 }

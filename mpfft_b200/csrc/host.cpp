@@ -1703,10 +1703,19 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
   const int T = 1 << S.lgT;
   S.nchunks = (int)(n / T);
   if (n >= 8) {
-    if (int e = upload(p, tier_leaf_slots(T, 1 << tier_leaf_lg(tier)), &S.slots[0])) return e;
+    auto slots = [&](int points) {  // those of four positions behind the others, where a tier has both
+      const int lg = tier_leaf_lg(tier, false), few = tier_leaf_lg(tier, true);
+      auto v = tier_leaf_slots(points, 1 << lg);
+      if (few != lg) {
+        const auto w = tier_leaf_slots(points, 1 << few);
+        v.insert(v.end(), w.begin(), w.end());
+      }
+      return v;
+    };
+    if (int e = upload(p, slots(T), &S.slots[0])) return e;
     S.slots[1] = S.slots[0];
     if (S.nchunks > 1) {
-      if (int e = upload(p, tier_leaf_slots(T / 2, 1 << tier_leaf_lg(tier)), &S.slots[1])) return e;
+      if (int e = upload(p, slots(T / 2), &S.slots[1])) return e;
       if (int e = upload(p, tree_chunks((int)n, T), &S.chunks)) return e;
     }
   }

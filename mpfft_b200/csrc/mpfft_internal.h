@@ -90,7 +90,7 @@ struct TierLeafSlot {
 struct TierTab {
   int N = 0, lgT = 0;
   int nchunks = 0;                        // N/T
-  const TierLeafSlot *slots[2] = {};      // base cases of a T- and a T/2-point tree
+  const TierLeafSlot *slots[2] = {};      // base cases of a T- and a T/2-point tree, behind each those of four positions
   const SrChunk *chunks = nullptr;        // by input class
   const double2 *tw = nullptr;            // (cos, sin) per level n = 8 .. N, tier_level_tw; planes by word
   size_t tw_len = 0;                      // entries of a plane
@@ -232,7 +232,7 @@ size_t tier_word_bytes(int tier);
 int tier_sub_max(int tier);
 int tier_tw_words(int tier);     // words of a twiddle's cos (and of its sin)
 int tier_pass_levels(int tier);  // levels per pass
-int tier_leaf_lg(int tier);      // lg of the positions of a base-case slot
+int tier_leaf_lg(int tier, bool few);  // lg of the positions of a base-case slot (few: for one chunk alone)
 // tw[h*len + level entry] = (cos, sin) word h of 2 pi k/n for every level n = 8
 // .. N, from w[(2h + part)*q + k'] of the N-point table (q = N/4)
 cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaStream_t s);

@@ -149,12 +149,12 @@ __global__ void __launch_bounds__(256) tier_queue_kernel(const QueueItem *__rest
       continue;
     }
     if (nl == 0) {
-      tier_sub_transform<NT, true>(S, A, tq_smem);
+      tier_sub_transform<NT, true, false>(S, A, tq_smem);
       continue;
     }
     for (A.c0 = 0; A.c0 < S.nchunks; ++A.c0) {
       __syncthreads();  // shared memory of the previous chunk is free
-      tier_sub_transform<NT, false>(S, A, tq_smem);
+      tier_sub_transform<NT, false, false>(S, A, tq_smem);
     }
     const int step = tier_upper_levels(nl, NT::kLevels);
     for (int done = 0; done < nl;) {

@@ -197,3 +197,36 @@ def test_tier_register_passes_inverse_scaled(M, orc, tier, n, batch):
     gr, gi = _from_words(O, y[0, :, -1] * n, prec), _from_words(O, y[1, :, -1] * n, prec)
     e = O.mp_errors(gr, gi, dr, di)["log2_rel"]
     assert e <= math.log2(8 * max(1.0, math.log2(n))) - bits, e
+
+
+@pytest.mark.parametrize("tier", ["ff", "dd", "qd"])
+@pytest.mark.parametrize("n,batch", [(8, 1301), (16, 1301), (32, 4801), (64, 1301), (128, 1301), (512, 1301), (1024, 1301),
+                                     (2048, 601), (8192, 151), (65536, 11)])
+def test_tier_single_signals_have_the_bits_of_a_batch(M, tier, n, batch):
+    """One signal (a kernel of its own where the launch has fewer chunks than the
+    GPU has SMs: other base cases, one level per pass) against the same signal in
+    batches that take several signals or chunks per CTA (the last CTA partly
+    filled) and several levels per pass."""
+    import torch
+
+    plan = M.MultiwordPlan(n, tier)
+    dtype = torch.float32 if tier == "ff" else torch.float64
+    eps = torch.finfo(dtype).eps
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.zeros((2, plan.words, batch, n), dtype=dtype, device="cuda")
+    x[:, 0] = 2 * torch.rand((2, batch, n), dtype=dtype, device="cuda", generator=gen) - 1
+    for h in range(1, plan.words):
+        x[:, h] = x[:, h - 1] * (0.4 * eps) * (torch.rand((2, batch, n), dtype=dtype, device="cuda", generator=gen) - 0.5)
+    y = torch.full_like(x, float("nan"))
+    s = torch.cuda.current_stream().cuda_stream
+    plan.execute_device(batch, x.data_ptr(), y.data_ptr(), stream=s)
+    assert bool(torch.isfinite(y).all())
+    for b in sorted({0, 1, 147 % batch, 148 % batch, batch // 2, *range(batch - 9, batch)}):
+        one = x[:, :, b].contiguous()
+        ref = torch.empty_like(one)
+        plan.execute_device(1, one.data_ptr(), ref.data_ptr(), stream=s)
+        assert torch.equal(y[:, :, b], ref), b
+    few = x[:, :, :min(146, batch)].contiguous()
+    out = torch.empty_like(few)
+    plan.execute_device(few.shape[2], few.data_ptr(), out.data_ptr(), stream=s)
+    assert torch.equal(out, y[:, :, :few.shape[2]])
