@@ -2669,9 +2669,8 @@ struct mpfft_batch_plan {
     mpfft_mp_plan *mp = nullptr;
     mpfft_d_plan *fp = nullptr;
   };
-  struct Queue {
-    int family = 0, L = 0;  // L: limb count of a limb queue
-    int threads = 256, sub = 0, ctas = 1;
+  struct Queue : QueueShape {
+    int sub = 0, ctas = 1;
     std::vector<unsigned long> sigs;  // largest first
     QueueItem *d_items = nullptr;
   };
@@ -2722,16 +2721,34 @@ struct mpfft_batch_plan {
 
 namespace mpfft {
 
+// Threads of a tier queue's CTAs.  A CTA takes one signal at a time, so short
+// signals need few threads, and more CTAs of them share an SM; long ones (several
+// chunks) make the end of the launch and take all the threads.  Measured (us, 64 /
+// 128 / 256 threads): double-double 256 points x 2000 37 / 65 / 100, 512 points
+// alone 14.4 / 12.5 / 12.8; quad-double 1024 points alone 84 / 57 / 44, x 2000 541 /
+// 501 / 570, 8192 points alone 935 / 574 / 419; float-float 1024 points x 2000 57 /
+// 61 / 98, 8192 points alone 84 / 49 / 39.
+static int tier_queue_threads(const mpfft_batch_plan *bp, const mpfft_batch_plan::Queue &Q, int sms) {
+  unsigned long most = 0;
+  for (unsigned long i : Q.sigs) most = std::max(most, bp->sig[i].n);
+  if (most > (unsigned long)Q.sub) return 256;
+  if (most <= 512) return most <= 256 ? 64 : 128;
+  return Q.sigs.size() > 2 * (size_t)sms ? 128 : 256;
+}
+
 // (Re)build a queue's tables and items for its current sub size, and its grid.
 static int batch_build_queue(mpfft_batch_plan *bp, int qi) {
   auto &Q = bp->queues[qi];
   std::vector<QueueItem> items;
+  Q.points = Q.chunk = 1;
   for (unsigned long i : Q.sigs) {
     auto &s = bp->sig[i];
     if (Q.family != kQueueLimbs) {
       s.fp = ft_cached(s.n, family_tier(Q.family), Q.sub);
       if (!s.fp) return g_err;
       bp->tabs[s.tab].ft = s.fp->tabs;
+      Q.points = std::max(Q.points, (long long)s.n);
+      Q.chunk = std::max(Q.chunk, 1 << (Q.family == kQueueDouble ? s.fp->tabs.d.lgT : s.fp->tabs.t.lgT));
     }
     items.push_back(QueueItem{bp->d_in + s.off, bp->d_out + s.off, bp->d_tabs + s.tab});
   }
@@ -2739,8 +2756,8 @@ static int batch_build_queue(mpfft_batch_plan *bp, int qi) {
   CUDA_TRY(cudaMemcpy(Q.d_items, items.data(), items.size() * sizeof(QueueItem), cudaMemcpyHostToDevice));
   int sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, bp->device));
-  CUDA_TRY(queue_prepare(Q.family, Q.L));
-  Q.ctas = (int)std::min<size_t>(Q.sigs.size(), (size_t)sms * queue_ctas_per_sm(Q.family, Q.L, Q.threads));
+  CUDA_TRY(queue_prepare(Q));
+  Q.ctas = (int)std::min<size_t>(Q.sigs.size(), (size_t)sms * queue_ctas_per_sm(Q));
   return MPFFT_OK;
 }
 
@@ -2757,8 +2774,7 @@ static int batch_capture(mpfft_batch_plan *bp) {
     const auto &Q = bp->queues[q];
     e = cudaStreamWaitEvent(bp->qstreams[q], bp->fork, 0);
     if (e == cudaSuccess)
-      e = queue_launch(Q.family, Q.L, Q.d_items, (int)Q.sigs.size(), bp->d_heads + q, Q.ctas, Q.threads, 1.0,
-                       bp->qstreams[q]);
+      e = queue_launch(Q, Q.d_items, (int)Q.sigs.size(), bp->d_heads + q, Q.ctas, 1.0, bp->qstreams[q]);
     if (e == cudaSuccess) e = cudaEventRecord(bp->joins[q], bp->qstreams[q]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(bp->stream, bp->joins[q], 0);
   }
@@ -2976,8 +2992,12 @@ MPFFT_API int mpfft_batch_plan_create(mpfft_batch_plan **plan, unsigned long cou
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&bp->stream, cudaStreamNonBlocking));
   CUDA_TRY(cudaEventCreateWithFlags(&bp->fork, cudaEventDisableTiming));
+  int sms = 0;
+  CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, bp->device));
   const auto tuned = tune_load();
   for (size_t q = 0; q < bp->queues.size(); ++q) {
+    if (family_tier(bp->queues[q].family) >= 0)
+      bp->queues[q].threads = tier_queue_threads(bp.get(), bp->queues[q], sms);
     cudaStream_t s;
     cudaEvent_t e;
     CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -3142,7 +3162,8 @@ MPFFT_API int mpfft_batch_autotune(mpfft_batch_plan *plan, int save) {
   for (size_t q = 0; q < plan->queues.size(); ++q) {
     auto &Q = plan->queues[q];
     std::vector<std::pair<int, int>> cand;
-    for (int th : {128, 256}) {
+    for (int th : {64, 128, 256}) {
+      if (th == 64 && family_tier(Q.family) < 0) continue;
       if (Q.family == kQueueLimbs) {
         cand.emplace_back(th, 0);
         continue;
@@ -3162,8 +3183,7 @@ MPFFT_API int mpfft_batch_autotune(mpfft_batch_plan *plan, int save) {
       for (int rep = 0; rep < 4; ++rep) {
         CUDA_TRY(cudaMemsetAsync(plan->d_heads + q, 0, sizeof(int), plan->stream));
         CUDA_TRY(cudaEventRecord(e0, plan->stream));
-        CUDA_TRY(queue_launch(Q.family, Q.L, Q.d_items, (int)Q.sigs.size(), plan->d_heads + q, Q.ctas, Q.threads, 1.0,
-                              plan->stream));
+        CUDA_TRY(queue_launch(Q, Q.d_items, (int)Q.sigs.size(), plan->d_heads + q, Q.ctas, 1.0, plan->stream));
         CUDA_TRY(cudaEventRecord(e1, plan->stream));
         CUDA_TRY(cudaEventSynchronize(e1));
         CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));

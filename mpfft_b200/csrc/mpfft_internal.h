@@ -262,16 +262,23 @@ struct QueueItem {
   const QueueTables *tab;
 };
 // Queue families: limb forms (one kernel per limb count), FP64, and the
-// compensated tiers.  A launch runs `ctas` persistent CTAs of `threads`
-// threads that pop items[0 .. nitems) through *head (an atomic counter the
-// caller zeroes before the launch) until the queue is empty; no CTA ever
-// waits for another.
+// compensated tiers.
 enum { kQueueLimbs = 0, kQueueDouble = 1, kQueueTierDD = 2, kQueueTierQD = 3, kQueueTierFF = 4 };
-cudaError_t queue_launch(int family, int L, const QueueItem *items, int nitems, int *head, int ctas, int threads,
-                         double scale, cudaStream_t s);
-// largest resident CTAs per SM of a family's kernel at `threads` threads
-int queue_ctas_per_sm(int family, int L, int threads);
-cudaError_t queue_prepare(int family, int L);  // kernel attributes, before any stream capture
+// Launch shape of a queue.
+struct QueueShape {
+  int family = 0, L = 0;   // L: limb count of a limb queue
+  int threads = 256;       // of a CTA
+  long long points = 1;    // floating forms: of the longest signal
+  int chunk = 1;           // floating forms: of the longest shared-memory chunk
+};
+// A launch runs `ctas` persistent CTAs that pop items[0 .. nitems) through *head
+// (an atomic counter the caller zeroes before the launch) until the queue is
+// empty; no CTA ever waits for another.
+cudaError_t queue_launch(const QueueShape &Q, const QueueItem *items, int nitems, int *head, int ctas, double scale,
+                         cudaStream_t s);
+// largest resident CTAs per SM of a queue's kernel
+int queue_ctas_per_sm(const QueueShape &Q);
+cudaError_t queue_prepare(const QueueShape &Q);  // kernel attributes, before any stream capture
 
 // Import -> transform -> export of device-resident MPFR fields with all
 // working storage in a file-scope device array (static_scratch.cu).  Returns an

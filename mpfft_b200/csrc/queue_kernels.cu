@@ -133,39 +133,56 @@ __device__ __forceinline__ void tier_queue_upper(const TierTab &S, typename NT::
     tier_upper_column<NT, R>(out, S, 1, lgu, 0, t >> lgu, t & ((1 << lgu) - 1), scale, false);
 }
 
-template <class NT>
-__global__ void __launch_bounds__(256) tier_queue_kernel(const QueueItem *__restrict__ items, int nitems, int *head,
-                                                         double scale) {
+// SHORT: no signal is longer than one chunk of 2^kLgFew points.  A CTA takes one
+// signal at a time, so short ones leave most of 256 threads idle: they run in
+// small CTAs (tier_queue_threads in host.cpp), several of which share an SM, one
+// level per pass, in a kernel without the code of longer signals.  Measured (2000
+// signals, us; one kernel for all lengths, 256 threads, one CTA per SM / this):
+// float-float 64 points 84 / 16, 512 points 123 / 27; double-double 102 / 29, 135
+// / 68; quad-double 221 / 78, 368 / 232.  The longer ones keep one CTA of all the
+// registers per SM: with two, of 128 registers, uniform batches are faster (double-double
+// 4096 points x 300 123 / 105 us) but the longest signals later (quad-double 8192
+// points alone 386 / 452 us; 2000 signals of 16 .. 8192 points in four forms 508 /
+// 806 us), and those end a mixed launch.
+template <class NT, bool SHORT>
+__global__ void __launch_bounds__(256, 1) tier_queue_kernel(const QueueItem *__restrict__ items, int nitems, int *head,
+                                                            double scale) {
   extern __shared__ __align__(16) double2 tq_smem[];
   __shared__ int slot;
   for (int i; (i = queue_next(head, &slot)) < nitems;) {
     const QueueItem it = items[i];
     const TierTab S = it.tab->ft.t;
     auto *out = static_cast<typename NT::W *>(it.out);
-    const int nl = 31 - __clz(S.nchunks);
-    TierArgs<NT> A{static_cast<const typename NT::W *>(it.in), out, 1, 0, 0, 1, NT::kLevels, scale, nl == 0, false, false};
+    const int nl = SHORT ? 0 : 31 - __clz(S.nchunks);
+    TierArgs<NT> A{static_cast<const typename NT::W *>(it.in), out, 1, 0, 0, 1, 1, scale, nl == 0, false, false};
     if (S.N < 8) {
       tier_tiny<NT>(S, A);
       continue;
     }
-    if (nl == 0) {
-      tier_sub_transform<NT, true, false>(S, A, tq_smem);
-      continue;
-    }
-    for (A.c0 = 0; A.c0 < S.nchunks; ++A.c0) {
-      __syncthreads();  // shared memory of the previous chunk is free
-      tier_sub_transform<NT, false, false>(S, A, tq_smem);
-    }
-    const int step = tier_upper_levels(nl, NT::kLevels);
-    for (int done = 0; done < nl;) {
-      __syncthreads();
-      const int r = min(step, nl - done), lgu = S.lgT + done - 1, cols = S.N >> (r + 1);
-      const double sc = done + r == nl ? scale : 1.0;
-      constexpr int R2 = NT::kLevels >= 2 ? 2 : 1, R3 = NT::kLevels >= 3 ? 3 : 1;
-      if (r == 3) tier_queue_upper<NT, R3>(S, out, lgu, cols, sc);
-      else if (r == 2) tier_queue_upper<NT, R2>(S, out, lgu, cols, sc);
-      else tier_queue_upper<NT, 1>(S, out, lgu, cols, sc);
-      done += r;
+    if constexpr (SHORT) {
+      tier_sub_transform<NT, true, true>(S, A, tq_smem);
+    } else {
+      // as many levels per pass as leave every thread a column
+      A.per = min(NT::kLevels, max(1, S.lgT - 1 - (31 - __clz(blockDim.x))));
+      if (nl == 0) {
+        tier_sub_transform<NT, true, false>(S, A, tq_smem);
+        continue;
+      }
+      for (A.c0 = 0; A.c0 < S.nchunks; ++A.c0) {
+        __syncthreads();  // shared memory of the previous chunk is free
+        tier_sub_transform<NT, false, false>(S, A, tq_smem);
+      }
+      const int step = tier_upper_levels(nl, NT::kLevels);
+      for (int done = 0; done < nl;) {
+        __syncthreads();
+        const int r = min(step, nl - done), lgu = S.lgT + done - 1, cols = S.N >> (r + 1);
+        const double sc = done + r == nl ? scale : 1.0;
+        constexpr int R2 = NT::kLevels >= 2 ? 2 : 1, R3 = NT::kLevels >= 3 ? 3 : 1;
+        if (r == 3) tier_queue_upper<NT, R3>(S, out, lgu, cols, sc);
+        else if (r == 2) tier_queue_upper<NT, R2>(S, out, lgu, cols, sc);
+        else tier_queue_upper<NT, 1>(S, out, lgu, cols, sc);
+        done += r;
+      }
     }
   }
 }
@@ -173,30 +190,36 @@ __global__ void __launch_bounds__(256) tier_queue_kernel(const QueueItem *__rest
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr size_t kQueueSmemBytes = 64 * 1024 + kOrderBytes;  // FP64 (4096 points) and every tier (64 KB planes)
+constexpr size_t kQueueSmemBytes = 64 * 1024 + kOrderBytes;  // most: FP64 (4096 points) and every tier (64 KB planes)
 
 template <int L>
 static const void *mp_queue_fn() {
   return (const void *)mp_queue_kernel<L>;
 }
 
-static const void *queue_fn(int family, int L) {
-  switch (family) {
+template <class NT>
+static const void *tier_queue_fn(const QueueShape &Q) {
+  if (Q.points == Q.chunk && Q.chunk <= 1 << NT::kLgFew) return (const void *)tier_queue_kernel<NT, true>;
+  return (const void *)tier_queue_kernel<NT, false>;
+}
+
+static const void *queue_fn(const QueueShape &Q) {
+  switch (Q.family) {
     case kQueueDouble:
       return (const void *)d_queue_kernel;
     case kQueueTierDD:
-      return (const void *)tier_queue_kernel<DDT>;
+      return tier_queue_fn<DDT>(Q);
     case kQueueTierQD:
-      return (const void *)tier_queue_kernel<QDT>;
+      return tier_queue_fn<QDT>(Q);
     case kQueueTierFF:
-      return (const void *)tier_queue_kernel<FFT_>;
+      return tier_queue_fn<FFT_>(Q);
     default:
       break;
   }
 #define MPFFT_Q_CASE(LL) \
   case LL:               \
     return mp_queue_fn<LL>();
-  switch (L) {
+  switch (Q.L) {
     MPFFT_Q_CASE(2) MPFFT_Q_CASE(3) MPFFT_Q_CASE(4) MPFFT_Q_CASE(5) MPFFT_Q_CASE(6) MPFFT_Q_CASE(7)
     MPFFT_Q_CASE(8) MPFFT_Q_CASE(9) MPFFT_Q_CASE(10) MPFFT_Q_CASE(11) MPFFT_Q_CASE(12) MPFFT_Q_CASE(13)
     MPFFT_Q_CASE(14) MPFFT_Q_CASE(15) MPFFT_Q_CASE(16) MPFFT_Q_CASE(17) MPFFT_Q_CASE(18) MPFFT_Q_CASE(19)
@@ -209,35 +232,35 @@ static const void *queue_fn(int family, int L) {
 #undef MPFFT_Q_CASE
 }
 
-static size_t queue_smem(int family, int L, int threads) {
-  return family == kQueueLimbs ? (size_t)L * threads * sizeof(uint32_t) : kQueueSmemBytes;
+static size_t queue_smem(const QueueShape &Q) {
+  if (Q.family == kQueueLimbs) return (size_t)Q.L * Q.threads * sizeof(uint32_t);
+  const int units = Q.family == kQueueTierDD ? DDT::kUnits : Q.family == kQueueTierQD ? QDT::kUnits : 1;
+  return (size_t)Q.chunk * units * sizeof(double2) + kOrderBytes;
 }
 
-cudaError_t queue_prepare(int family, int L) {
-  const void *fn = queue_fn(family, L);
+cudaError_t queue_prepare(const QueueShape &Q) {
+  const void *fn = queue_fn(Q);
   if (!fn) return cudaErrorInvalidValue;
-  if (family == kQueueLimbs) return cudaSuccess;
+  if (Q.family == kQueueLimbs) return cudaSuccess;
   return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kQueueSmemBytes);
 }
 
-int queue_ctas_per_sm(int family, int L, int threads) {
-  const void *fn = queue_fn(family, L);
+int queue_ctas_per_sm(const QueueShape &Q) {
+  const void *fn = queue_fn(Q);
   int n = 0;
-  if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, queue_smem(family, L, threads)) !=
-                 cudaSuccess)
-    return 1;
+  if (!fn || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, Q.threads, queue_smem(Q)) != cudaSuccess) return 1;
   return std::max(1, n);
 }
 
-cudaError_t queue_launch(int family, int L, const QueueItem *items, int nitems, int *head, int ctas, int threads,
-                         double scale, cudaStream_t s) {
+cudaError_t queue_launch(const QueueShape &Q, const QueueItem *items, int nitems, int *head, int ctas, double scale,
+                         cudaStream_t s) {
   if (nitems <= 0) return cudaSuccess;
-  const void *fn = queue_fn(family, L);
+  const void *fn = queue_fn(Q);
   if (!fn) return cudaErrorInvalidValue;
   void *args_mp[] = {(void *)&items, (void *)&nitems, (void *)&head};
   void *args_fp[] = {(void *)&items, (void *)&nitems, (void *)&head, (void *)&scale};
-  return cudaLaunchKernel(fn, dim3(ctas), dim3(threads), family == kQueueLimbs ? args_mp : args_fp,
-                          queue_smem(family, L, threads), s);
+  return cudaLaunchKernel(fn, dim3(ctas), dim3(Q.threads), Q.family == kQueueLimbs ? args_mp : args_fp, queue_smem(Q),
+                          s);
 }
 
 }  // namespace mpfft

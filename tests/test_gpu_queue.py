@@ -195,3 +195,52 @@ def test_queue_groups_of_ragged_sizes(M, orc, count):
     M.MpPlan(n, p, float_tiers=False).execute(count, xr.ptr, xi.ptr, zr.ptr, zi.ptr)
     assert L.orc_mp_count_diff(yr.ptr, zr.ptr, n * count) == 0
     assert L.orc_mp_count_diff(yi.ptr, zi.ptr, n * count) == 0
+
+
+class _Arena:
+    """Device memory of a batch plan as an array, for torch.as_tensor."""
+
+    def __init__(self, ptr, nbytes):
+        self.__cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (ptr, False), "version": 3}
+
+
+@pytest.mark.parametrize("tier,prec", [("ff", 24), ("dd", 106), ("qd", 212)])
+@pytest.mark.parametrize("lengths,copies,threads", [
+    ([1, 2, 4, 8, 16], 3, 64), ([8, 32, 64, 128, 256], 70, 64), ([512], 1, 128), ([16, 512, 64, 4], 90, 128),
+    ([1024, 8, 512], 2, 256), ([1024, 256], 150, 128), ([8, 4096, 64, 8192, 1024], 2, 256)])
+def test_tier_queues_fit_their_signals(M, monkeypatch, tmp_path, tier, prec, lengths, copies, threads):
+    """Short signals run in CTAs of as many threads as they have work for (several
+    CTAs share an SM), long ones in CTAs of 256; every signal has the bits of its
+    single call, whichever kernel and levels per pass its queue takes."""
+    import torch
+
+    monkeypatch.setenv("MPFFT_AUTOTUNE_FILE", str(tmp_path / "none.json"))
+    ns = lengths * copies
+    plan = M.BatchPlan(ns, [prec] * len(ns), float_tiers="native")
+    (q,) = plan.queues()
+    assert q["signals"] == len(ns) and q["threads"] == threads
+    a, b, nbytes = plan.arenas()
+    ain, aout = (torch.as_tensor(_Arena(p, nbytes), device="cuda") for p in (a, b))
+    dtype = torch.float32 if tier == "ff" else torch.float64
+    eps = torch.finfo(dtype).eps
+    gen = torch.Generator(device="cuda").manual_seed(len(ns) + prec)
+    parts = []
+    for i, n in enumerate(ns):
+        _, words, off, size = plan.signal_format(i)
+        x = ain[off:off + size].view(dtype).view(2, words, n)
+        x[:, 0] = 2 * torch.rand((2, n), dtype=dtype, device="cuda", generator=gen) - 1
+        for h in range(1, words):
+            x[:, h] = x[:, h - 1] * (0.4 * eps) * (torch.rand((2, n), dtype=dtype, device="cuda", generator=gen) - 0.5)
+        y = aout[off:off + size].view(dtype).view(2, words, n)
+        y.fill_(float("nan"))
+        parts.append((x, y))
+    torch.cuda.synchronize()
+    s = torch.cuda.current_stream().cuda_stream
+    plan.execute_device(s)
+    singles = {n: M.MultiwordPlan(n, tier) for n in set(ns)}
+    for i in sorted({*range(0, len(ns), 7), *range(len(lengths)), len(ns) - 1}):
+        x, y = parts[i]
+        ref = torch.empty_like(x)
+        singles[ns[i]].execute_device(1, x.data_ptr(), ref.data_ptr(), stream=s)
+        assert torch.equal(y, ref), (i, ns[i])
+    assert all(bool(torch.isfinite(y).all()) for _, y in parts)
