@@ -128,3 +128,36 @@ def test_d_register_passes_bitexact(M, orc, n, batch, inverse):
         else:
             er, ei = f(x[0, b].copy(), x[1, b].copy())
         assert _bits_equal(y[0, b], er) and _bits_equal(y[1, b], ei), b
+
+
+@pytest.mark.parametrize("n,batch", [(1, 5000), (2, 3001), (4, 2049), (16, 331), (32, 4801), (64, 1201), (128, 2371),
+                                     (256, 601), (512, 2401), (1024, 1187), (2048, 601), (8192, 75), (65536, 10),
+                                     (131072, 11)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_d_several_signals_or_chunks_per_cta(M, orc, n, batch, inverse):
+    """Batches in which a CTA takes several signals (the last CTA partly filled) or
+    several chunks of one signal: every signal has the bits of its single call
+    (one per CTA), and three of them those of the reference's transform."""
+    import torch
+
+    gen = torch.Generator(device="cuda").manual_seed(n + batch)
+    x = 2 * torch.rand((2, batch, n), dtype=torch.float64, device="cuda", generator=gen) - 1
+    y, ref = torch.full_like(x, float("nan")), torch.empty_like(x)
+    plan = M.DPlan(n)
+    s = torch.cuda.current_stream().cuda_stream
+    plan.execute_device(batch, x.data_ptr(), y.data_ptr(), scaled=inverse, inverse=inverse, stream=s)
+    for b in range(batch):
+        one = x[:, b].contiguous()
+        out = torch.empty_like(one)
+        plan.execute_device(1, one.data_ptr(), out.data_ptr(), scaled=inverse, inverse=inverse, stream=s)
+        ref[:, b] = out
+    assert torch.equal(y.view(torch.int64), ref.view(torch.int64))
+    h, f = x.cpu().numpy(), orc.DFFT(n)
+    for b in (0, batch // 2, batch - 1):
+        r, i = h[0, b].copy(), h[1, b].copy()
+        if inverse:
+            ei, er = f(i, r)
+            er, ei = er / n, ei / n
+        else:
+            er, ei = f(r, i)
+        assert _bits_equal(y[0, b].cpu().numpy(), er) and _bits_equal(y[1, b].cpu().numpy(), ei), b
