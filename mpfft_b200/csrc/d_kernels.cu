@@ -61,18 +61,16 @@ __global__ void __launch_bounds__(256, 2) d_upper_kernel(double *__restrict__ y,
                     swap_out != 0);
 }
 
-__global__ void __launch_bounds__(256) d_level_tw_kernel(const double *__restrict__ wr, const double *__restrict__ wi,
-                                                         int N, double2 *__restrict__ tw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of the table
-  if (i >= N / 2 - 8) return;
+__global__ void __launch_bounds__(256) d_level_tw_kernel(int N, double2 *tw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of a level below N
+  if (i >= N / 4 - 8) return;
   const int q = 1 << (31 - __clz(i + 8));  // n/4 of its level: entries q-8 .. 2q-9
   const int k = i + 8 - q;
-  const size_t kn = (size_t)k * (N / (4 * q));
-  tw[i] = make_double2(wr[kn], wi[kn]);
+  tw[i] = tw[sr_level_tw(N) + (size_t)k * (N / (4 * q))];
 }
 
-cudaError_t d_build_level_tw(const double *wr, const double *wi, int N, double2 *tw, cudaStream_t s) {
-  d_level_tw_kernel<<<(N / 2 + 255) / 256, 256, 0, s>>>(wr, wi, N, tw);
+cudaError_t d_build_level_tw(int N, double2 *tw, cudaStream_t s) {
+  if (N > 32) d_level_tw_kernel<<<(N / 4 - 8 + 255) / 256, 256, 0, s>>>(N, tw);
   return cudaGetLastError();
 }
 

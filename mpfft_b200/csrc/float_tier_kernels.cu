@@ -54,19 +54,16 @@ __global__ void __launch_bounds__(256) tier_upper_kernel(typename NT::W *__restr
                            swap_out != 0);
 }
 
-__global__ void __launch_bounds__(256) tier_tw_kernel(const double *__restrict__ w, int words, int N,
-                                                      double2 *__restrict__ tw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of a plane
-  const int len = N / 2 - 2;
-  if (i >= len) return;
+__global__ void __launch_bounds__(256) tier_tw_kernel(int words, int N, double2 *tw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // entry of a level below N, in each plane
+  if (i >= N / 4 - 2) return;
   const int q = 1 << (31 - __clz(i + 2));  // n/4 of its level: entries q-2 .. 2q-3
-  const size_t kn = (size_t)(i + 2 - q) * (N / (4 * q)), n4 = (size_t)N / 4;
-  for (int h = 0; h < words; ++h)
-    tw[(size_t)h * len + i] = make_double2(w[(size_t)(2 * h) * n4 + kn], w[(size_t)(2 * h + 1) * n4 + kn]);
+  const size_t kn = (size_t)(i + 2 - q) * (N / (4 * q)), len = (size_t)N / 2 - 2;
+  for (int h = 0; h < words; ++h) tw[h * len + i] = tw[h * len + tier_level_tw(N) + kn];
 }
 
-cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaStream_t s) {
-  tier_tw_kernel<<<(N / 2 + 255) / 256, 256, 0, s>>>(w, words, N, tw);
+cudaError_t tier_build_tw(int words, int N, double2 *tw, cudaStream_t s) {
+  if (N > 8) tier_tw_kernel<<<(N / 4 - 2 + 255) / 256, 256, 0, s>>>(words, N, tw);
   return cudaGetLastError();
 }
 

@@ -1479,27 +1479,21 @@ static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
     }
   }
   // twiddles exactly as the reference lut() (serial_d_fft6.c:52-62)
-  const unsigned long q = n / 4;
-  std::vector<double> wr(q ? q : 1), wi(q ? q : 1);
-  for (unsigned long k = 0; k < q; ++k) {
-    wr[k] = cos(2. * M_PI * k / n);
-    wi[k] = sin(2. * M_PI * k / n);
-  }
+  const unsigned long q = n > 16 ? n / 4 : 0;
+  std::vector<double2> w(q);
+  for (unsigned long k = 0; k < q; ++k) w[k] = make_double2(cos(2. * M_PI * k / n), sin(2. * M_PI * k / n));
   S.K.c8 = cos(2. * M_PI * 1 / 8);
   S.K.c16a = cos(2. * M_PI * 1 / 16);
   S.K.c16b = cos(2. * M_PI * 1 / 16) - cos(2. * M_PI * 3 / 16);
   S.K.c16c = cos(2. * M_PI * 3 / 16);
   S.K.c16d = cos(2. * M_PI * 1 / 16) + cos(2. * M_PI * 3 / 16);
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
-  if (n > 16) {  // the levels' twiddles, gathered from that table on the device
-    // (one allocation, the source table behind the levels: freeing it here would synchronise the device)
+  if (n > 16) {  // that table is the last level; the others are gathered from it on the device
     double2 *d_tw = nullptr;
-    CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2) + 2 * q * sizeof(double)));
+    CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2)));
     p->dev_allocs.push_back(d_tw);
-    double *d_w = reinterpret_cast<double *>(d_tw + (n / 2 - 8));
-    CUDA_TRY(cudaMemcpyAsync(d_w, wr.data(), q * sizeof(double), cudaMemcpyHostToDevice, p->stream));
-    CUDA_TRY(cudaMemcpyAsync(d_w + q, wi.data(), q * sizeof(double), cudaMemcpyHostToDevice, p->stream));
-    CUDA_TRY(d_build_level_tw(d_w, d_w + q, (int)n, d_tw, p->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_tw + sr_level_tw((int)n), w.data(), q * sizeof(double2), cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(d_build_level_tw((int)n, d_tw, p->stream));
     CUDA_TRY(cudaStreamSynchronize(p->stream));
     S.tw = d_tw;
   }
@@ -1721,7 +1715,7 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
   }
   const int K = tier_tw_words(tier);
   const unsigned long q = std::max<unsigned long>(1, n / 4);
-  std::vector<double> w((size_t)2 * K * q);  // [word][cos, sin][k]
+  std::vector<double2> w((size_t)K * q);  // [word][k] (cos, sin)
   parallel_for((long)q, 64, [&](long a, long b) {
     mpfr_t th, c, s;
     mpfr_init2(th, 360);
@@ -1733,11 +1727,10 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
       mpfr_div_ui(th, th, n, MPFR_RNDN);
       mpfr_sin_cos(s, c, th, MPFR_RNDN);
       for (int h = 0; h < K; ++h) {  // exact remainders at 320 bits
-        double *wc = &w[(size_t)(2 * h) * q + k], *ws = wc + q;
-        *wc = mpfr_get_d(c, MPFR_RNDN);
-        mpfr_sub_d(c, c, *wc, MPFR_RNDN);
-        *ws = mpfr_get_d(s, MPFR_RNDN);
-        mpfr_sub_d(s, s, *ws, MPFR_RNDN);
+        double2 &t = w[(size_t)h * q + k];
+        t = make_double2(mpfr_get_d(c, MPFR_RNDN), mpfr_get_d(s, MPFR_RNDN));
+        mpfr_sub_d(c, c, t.x, MPFR_RNDN);
+        mpfr_sub_d(s, s, t.y, MPFR_RNDN);
       }
     }
     mpfr_clear(th);
@@ -1746,14 +1739,14 @@ static int d_plan_init_tier(mpfft_d_plan *p, unsigned long n, int tier, int sub_
     mpfr_free_cache();
   });
   CUDA_TRY(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
-  if (n >= 8) {  // the levels' twiddles, gathered from that table on the device (one allocation, see d_plan_init)
+  if (n >= 8) {  // that table is the last level of each plane; the others are gathered from it on the device
     S.tw_len = n / 2 - 2;
     double2 *d_tw = nullptr;
-    CUDA_TRY(cudaMalloc(&d_tw, S.tw_len * K * sizeof(double2) + w.size() * sizeof(double)));
+    CUDA_TRY(cudaMalloc(&d_tw, S.tw_len * K * sizeof(double2)));
     p->dev_allocs.push_back(d_tw);
-    double *d_w = reinterpret_cast<double *>(d_tw + S.tw_len * K);
-    CUDA_TRY(cudaMemcpyAsync(d_w, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, p->stream));
-    CUDA_TRY(tier_build_tw(d_w, K, (int)n, d_tw, p->stream));
+    CUDA_TRY(cudaMemcpy2DAsync(d_tw + (S.tw_len - q), S.tw_len * sizeof(double2), w.data(), q * sizeof(double2),
+                               q * sizeof(double2), K, cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(tier_build_tw(K, (int)n, d_tw, p->stream));
     CUDA_TRY(cudaStreamSynchronize(p->stream));
     S.tw = d_tw;
   }

@@ -216,8 +216,9 @@ cudaError_t mp_export_launch(const uint32_t *planes, int N, int B, int L, const 
 // out[m][c][r][e] = in[m][r][c][e]: nmat matrices of R x C elements of E words
 cudaError_t transpose_launch(const uint32_t *in, uint32_t *out, long long nmat, long long R, long long C, int E,
                              cudaStream_t s);
-// tw[sr_level_tw(n) + k] = (wr, wi)[k*(N/n)] for every level n = 32 .. N
-cudaError_t d_build_level_tw(const double *wr, const double *wi, int N, double2 *tw, cudaStream_t s);
+// the levels n = 32 .. N/2 of a table from its level N: tw[sr_level_tw(n) + k] =
+// tw[sr_level_tw(N) + k*(N/n)]
+cudaError_t d_build_level_tw(int N, double2 *tw, cudaStream_t s);
 // FP64 layout: word (c, b, p) at base[(c*B + b)*N + p]  (signal-contiguous)
 // swap_in / swap_out: read the input's / write the output's real and imaginary
 // planes exchanged (both: the unscaled inverse, swap(FFT(swap(x))))
@@ -233,9 +234,8 @@ int tier_sub_max(int tier);
 int tier_tw_words(int tier);     // words of a twiddle's cos (and of its sin)
 int tier_pass_levels(int tier);  // levels per pass
 int tier_leaf_lg(int tier, bool few);  // lg of the positions of a base-case slot (few: for one chunk alone)
-// tw[h*len + level entry] = (cos, sin) word h of 2 pi k/n for every level n = 8
-// .. N, from w[(2h + part)*q + k'] of the N-point table (q = N/4)
-cudaError_t tier_build_tw(const double *w, int words, int N, double2 *tw, cudaStream_t s);
+// the levels n = 8 .. N/2 of each plane of a tier's table from its level N
+cudaError_t tier_build_tw(int words, int N, double2 *tw, cudaStream_t s);
 // split step of the FP64 real transforms (n = 2M real points), d_kernels.cu
 cudaError_t d_real_split(bool forward, const double *in, double *out, int M, int B, const double *wc,
                          const double *ws, double scale, cudaStream_t s);

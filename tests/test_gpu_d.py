@@ -161,3 +161,21 @@ def test_d_several_signals_or_chunks_per_cta(M, orc, n, batch, inverse):
         else:
             er, ei = f(r, i)
         assert _bits_equal(y[0, b].cpu().numpy(), er) and _bits_equal(y[1, b].cpu().numpy(), ei), b
+
+
+@pytest.mark.parametrize("form,n,bytes_per_point", [("fp64", 1 << 22, 8), ("dd", 1 << 20, 16), ("qd", 1 << 19, 32),
+                                                    ("ff", 1 << 21, 8)])
+def test_plan_holds_its_twiddles_once(M, form, n, bytes_per_point):
+    """Device memory of a plan: the twiddles of all levels (N/2 complex values of the
+    form's words) and tables that do not grow with them; freed with the plan."""
+    import torch
+
+    torch.cuda.synchronize()
+    make = (lambda k: M.DPlan(k)) if form == "fp64" else (lambda k: M.MultiwordPlan(k, form))
+    make(64).close()
+    free = torch.cuda.mem_get_info()[0]
+    plan = make(n)
+    held = free - torch.cuda.mem_get_info()[0]
+    assert bytes_per_point * n <= held + (2 << 20) and held <= bytes_per_point * n + (6 << 20), held
+    plan.close()
+    assert free - torch.cuda.mem_get_info()[0] <= 2 << 20
