@@ -393,8 +393,9 @@ size_t mpfft_static_scratch_bytes(void);
  * butterfly launch (after the one leaf launch).  Returns the level count. */
 int mpfft_mp_plan_schedule(const mpfft_mp_plan *plan, int *level_n, int *level_nodes, int max_levels);
 /* The transform of mpfft_mp_execute_device run level by level, every launch
- * bracketed by CUDA events on `stream` (the untimed call runs several levels
- * per launch where that is faster; the results are the same);
+ * bracketed by CUDA events on `stream`, to tell the time by level (where that is
+ * faster the untimed call runs several levels per launch, and from 35 limbs all
+ * of them; the results are the same);
  * launch_ms[0] = leaf launch, launch_ms[1+i] = level i.  A level
  * that ran in one launch with level i-1 (large batches: two levels per
  * launch) reads 0 and the launch's time is in level i-1's entry.  Synchronous. */

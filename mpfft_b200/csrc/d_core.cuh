@@ -1,8 +1,8 @@
 // Device functions of the FP64 conjugate-pair split-radix kernels: the
 // reference's n=8 and n=16 base cases, the 4m2a butterfly, passes of up to
-// three levels in registers and one CTA's shared-memory sub-transforms.  Shared by the per-launch kernels
-// (d_kernels.cu) and the persistent work-queue kernels (queue_kernels.cu);
-// every file that includes it is compiled with --fmad=false so that no
+// three levels in registers and one CTA's shared-memory sub-transforms.
+// Shared by the per-launch kernels (d_kernels.cu) and the persistent
+// work-queue kernels (queue_kernels.cu); every file that includes it is compiled with --fmad=false so that no
 // multiply-add is contracted and results stay bit-identical to the reference.
 #pragma once
 

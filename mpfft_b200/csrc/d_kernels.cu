@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256) d_tiny_kernel(const __grid_constant__ DSu
 // R levels above the sub-transforms: one thread per column (d_upper_column),
 // consecutive threads consecutive k of one chunk of one signal.  Memory-bound:
 // three levels cross memory once instead of three times (one 2^20-point signal
-// 100 -> 39 us, five launches instead of nine).
+// 100 -> 39 us, four launches instead of nine).
 template <int R>
 __global__ void __launch_bounds__(256, 2) d_upper_kernel(double *__restrict__ y, int N, int B, int lgu, int lgnch,
                                                          const double2 *__restrict__ tw, double scale, int swap_out) {

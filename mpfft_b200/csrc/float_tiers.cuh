@@ -534,7 +534,9 @@ __device__ __forceinline__ void tier_put(typename NT::W *re, typename NT::W *im,
 constexpr int kOrder = 272, kOrderPairs = 176;  // up to 256 chunks (16 of 4096 points), 171 nodes and 85 pairs
 constexpr size_t kOrderBytes = kOrder * sizeof(uint16_t);
 
-__device__ __forceinline__ uint16_t *tier_order(double2 *sm, int units) { return reinterpret_cast<uint16_t *>(sm + units); }
+__device__ __forceinline__ uint16_t *tier_order(double2 *sm, int units) {
+  return reinterpret_cast<uint16_t *>(sm + units);
+}
 
 __device__ __forceinline__ void tier_fill_order(uint16_t *order, int chunks) {
   for (int m = threadIdx.x; m < chunks; m += blockDim.x) {
@@ -610,7 +612,8 @@ __device__ __forceinline__ void tier_sub_transform(const TierTab &S, const TierA
     __syncthreads();
     if (FEW) tier_pass<NT, 1, SINGLE, true>(S, A, sm, done - 1, last);
     else if (NT::kLevels == 3 && r == 3) tier_pass<NT, NT::kLevels, SINGLE, false>(S, A, sm, done - 1, last);
-    else if (NT::kLevels >= 2 && r == 2) tier_pass<NT, NT::kLevels >= 2 ? 2 : 1, SINGLE, false>(S, A, sm, done - 1, last);
+    else if (NT::kLevels >= 2 && r == 2)
+      tier_pass<NT, NT::kLevels >= 2 ? 2 : 1, SINGLE, false>(S, A, sm, done - 1, last);
     else tier_pass<NT, 1, SINGLE, false>(S, A, sm, done - 1, last);
     done += r;
   }

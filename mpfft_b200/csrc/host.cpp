@@ -1492,7 +1492,8 @@ static int d_plan_init(mpfft_d_plan *p, unsigned long n, int sub_max) {
     double2 *d_tw = nullptr;
     CUDA_TRY(cudaMalloc(&d_tw, (n / 2 - 8) * sizeof(double2)));
     p->dev_allocs.push_back(d_tw);
-    CUDA_TRY(cudaMemcpyAsync(d_tw + sr_level_tw((int)n), w.data(), q * sizeof(double2), cudaMemcpyHostToDevice, p->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_tw + sr_level_tw((int)n), w.data(), q * sizeof(double2), cudaMemcpyHostToDevice,
+                             p->stream));
     CUDA_TRY(d_build_level_tw((int)n, d_tw, p->stream));
     CUDA_TRY(cudaStreamSynchronize(p->stream));
     S.tw = d_tw;
@@ -1679,7 +1680,7 @@ static int d_execute_impl(mpfft_d_plan *p, unsigned long batch, const double *in
 }
 
 // Compensated-tier plan (double-double, quad-double, float-float): the same
-// tree, cut at T = min(n, tier_sub_max) points, base cases of at most 4
+// tree, cut at T points (sub_lg, at most tier_sub_max), base cases of at most 4
 // points; cos and sin of 2 pi k/n computed by MPFR at 320 bits and split into
 // the tier's words (each the nearest double to what the words above leave;
 // float-float keeps one double: its products are formed in FP64).

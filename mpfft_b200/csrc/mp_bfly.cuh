@@ -155,9 +155,9 @@ __device__ __forceinline__ void combine(uint32_t *u0, uint32_t *u1, uint32_t *zp
 // slot for the side's first product (words ps apart); twp: packed twiddles of
 // all k ([k][cos, cos+sin, |cos-sin|][Lp]: a row is read four limbs per load, for
 // one row a product instead of L strided words; N=1024, batch 2048, 33 limbs: 2357
-// -> 2288 us, 65536 points, batch 24, 34 limbs: 3608 -> 3494 us).  The merged products are stored with L2 priority
-// evict_last (a fused thread of mp_level_pair_kernel reads them back only
-// after two more butterflies).  mp_bfly_one below spells out the same steps
+// -> 2288 us, 65536 points, batch 24, 34 limbs: 3608 -> 3494 us).  The merged
+// products are stored with L2 priority evict_last (a fused thread of
+// mp_level_pair_kernel reads them back only after two more butterflies).  mp_bfly_one below spells out the same steps
 // inline (its register allocation at 33 limbs spills less that way); the
 // kernels built on each are checked to be bit-identical.
 template <int L>

@@ -7,10 +7,10 @@
 // same tree is executed breadth-first: one launch runs every leaf (n = 4, 2 or
 // 1), then one launch per node size n = 8, 16, ..., N runs every butterfly of
 // every node of that size (for large batches one launch per two node sizes,
-// mp_level_pair_kernel; in between several per launch, mp_smem_kernels.cu).  All nodes of one size are independent, so each
-// launch is one flat grid over (node, k, signal); consecutive threads are
-// consecutive signals of a batch (or consecutive k for a single signal),
-// which makes every limb-plane access a coalesced 128-byte transaction and,
+// mp_level_pair_kernel; in between several per launch, mp_smem_kernels.cu).
+// All nodes of one size are independent, so each launch is one flat grid over
+// (node, k, signal); consecutive threads are consecutive signals of a batch
+// (or consecutive k for a single signal), which makes every limb-plane access a coalesced 128-byte transaction and,
 // for batches, makes the twiddle operand warp-uniform.
 //
 // Data layout (limb planes): word (c, i, p, b) of a batch of B signals of
@@ -208,6 +208,10 @@ struct CombineChains {
   }
 };
 
+// (Up to 14 limbs the batches that would fill these launches run in tiles,
+// mp_tile_used; timed calls, which tell the time by level, reach the pair kernel
+// of those counts, and the figures of 9 limbs below are of such launches.)
+
 // Limb counts up to which combine_pair's limb loop is unrolled; above, the
 // unrolled loop's register demand next to the 128-register product costs more
 // than it saves, and the rolled loop reads the Z slots through ld_hint (kept
@@ -270,12 +274,6 @@ constexpr int pair_min_blocks() {
   return L >= 31 ? 3 : level_min_blocks<L>();
 }
 
-// one word of global memory to shared memory, asynchronously
-__device__ __forceinline__ void cp_async_word(uint32_t *dst, const uint32_t *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const uint32_t *a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 
 constexpr int kPairThreads = 128;
@@ -285,8 +283,10 @@ constexpr int kPairThreads = 128;
 // step needs it (mp_bfly_steps).  With three CTAs per SM a warp that waits for
 // its loads is rarely covered by the other two of its scheduler; from 31 limbs
 // that outweighs the copies (N=1024, batch 2048, us per batch, read / fetched:
-// 9 limbs 436 / 452, 17 limbs 906 / 911, 25 limbs 1462 / 1444, 33 limbs 2285 / 2211;
-// 65536 points, batch 24, 34 limbs 3500 / 3404).
+// 9 limbs 436 / 452, 17 limbs 906 / 911, 33 limbs 2285 / 2211; 65536 points, batch
+// 24, 34 limbs 3500 / 3404).  Below, with four CTAs, it does so at most counts from
+// 21 (21 limbs 1156 / 1118, 25 limbs 1443 / 1422, 30 limbs 2063 / 1873) but not at
+// all (28 limbs 1721 / 1746).
 template <int L>
 constexpr bool pair_async = L >= 31;
 template <int L>
@@ -314,7 +314,7 @@ __device__ __forceinline__ void mp_pair_steps(uint32_t *p, size_t qB, size_t pla
   auto slot = [&](int s) { return p + (size_t)(s < 2 ? 2 + s : 3 + (s >> 1) + 2 * (s & 1)) * qB; };
   auto fetch = [&](uint32_t *dst, const uint32_t *src) {
 #pragma unroll
-    for (int i = 0; i < L; ++i) cp_async_word(dst + (size_t)i * ps, src + (size_t)i * plane);
+    for (int i = 0; i < L; ++i) cp_async4(dst + (size_t)i * ps, src + (size_t)i * plane);
   };
   fetch(Sr, slot(first));
   fetch(Si, slot(first) + cim);

@@ -49,6 +49,14 @@ __device__ __forceinline__ uint32_t ld_hint(const uint32_t *a, uint64_t pol) {
   return v;
 }
 
+// one word of global memory to shared memory, asynchronously (cp_async_wait:
+// this thread's copies so far have arrived)
+__device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // one step of a carry chain: returns a + b + c (mod 2^32), c <- carry out
 __device__ __forceinline__ uint32_t addc(uint32_t a, uint32_t b, uint32_t &c) {
   const uint64_t t = (uint64_t)a + b + c;

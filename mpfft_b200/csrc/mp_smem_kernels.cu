@@ -36,7 +36,7 @@ namespace mpfft {
 
 // Tile size (complex numbers) by limb count, threads per CTA and the CTAs per
 // SM the register allocation must allow.  The tile's planes take 8L bytes per
-// number, so 227 KB hold 3152 numbers at 9 limbs and 860 at 33.  One thread per
+// number, so 227 KB hold 3228 numbers at 9 limbs and 880 at 33.  One thread per
 // four numbers: a level keeps between half and all of P/2 sides busy, so more
 // threads idle at the barriers and take the registers that let products
 // overlap.  Measured (us, N=1024, batch 2048; tile/threads): 9 limbs 512/128
@@ -299,11 +299,6 @@ __device__ __forceinline__ void tile_leaves(const MpTile &A, int chunk, int b0, 
   }
 }
 
-__device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-
 // Butterflies r0 .. r0+nr-1 of every node of one level.  t: lg of the number of
 // chunks of the node size in the tile; cnt nodes, node j < listed at chunk
 // nodes[j], the one after them at the last chunk.  last: outputs to global memory.
@@ -391,7 +386,7 @@ __global__ void __launch_bounds__(tile_threads<L, WIDE>(), smem_min_blocks<L, WI
         for (int x = 0; x < 2 * L; ++x) cp_async4(d + x * P, p + x * plane);
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    cp_async_wait();
   }
   // phase 0 of a first-launch level: the butterflies with products, r = k = 1 .. qr-1;
   // phase 1: k = 0

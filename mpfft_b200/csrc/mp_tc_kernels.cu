@@ -68,9 +68,9 @@ namespace mpfft {
 constexpr int kTcRows = 128;     // signals per CTA (MMA M)
 constexpr int kTcThreads = 256;  // two per signal
 
-// Tensor memory per CTA: two 128-column accumulators (one stage).  At least 80 KB of shared memory per CTA keeps
-// a third CTA off the SM, so 2 x 256 of the 512 columns suffice and an
-// allocation never waits.  (Measured: four CTAs per SM with one accumulator
+// Tensor memory per CTA: two 128-column accumulators (one stage).  At least
+// 80 KB of shared memory per CTA keeps a third CTA off the SM, so 2 x 256 of the
+// 512 columns suffice and an allocation never waits.  (Measured: four CTAs per SM with one accumulator
 // each and at most 128 registers per thread was slower from 65 limbs up.)
 constexpr uint32_t kTcMinSmem = 80u * 1024u;
 constexpr uint32_t kTcTmemCols = 256;
@@ -78,8 +78,9 @@ constexpr uint32_t kTcTmemCols = 256;
 constexpr uint32_t kTcIdesc = (2u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
 __device__ int g_tc_error = 0;  // first error code of any CTA (0 = none)
-// Limit of each wait on this CTA's own MMAs, in ns of %globaltimer.  Only a
-// test changes it (mpfft_diag_tc_set_wait_limit), to make the waits give up.
+// Limit of each wait -- on this CTA's own MMAs, and on the flags of the items
+// whose outputs an item reads -- in ns of %globaltimer.  Only a test changes it
+// (mpfft_diag_tc_set_wait_limit), to make the waits give up.
 __device__ unsigned long long g_tc_wait_ns = 2000000000ull;
 // Limit of the wait that drains a CTA's MMAs before it frees tensor memory
 // after another wait gave up; not affected by the test setting.

@@ -90,7 +90,8 @@ struct TierLeafSlot {
 struct TierTab {
   int N = 0, lgT = 0;
   int nchunks = 0;                        // N/T
-  const TierLeafSlot *slots[2] = {};      // base cases of a T- and a T/2-point tree, behind each those of four positions
+  const TierLeafSlot *slots[2] = {};      // base cases of a T- and a T/2-point tree (behind each, those of
+                                          // tier_leaf_lg(tier, true) where they differ)
   const SrChunk *chunks = nullptr;        // by input class
   const double2 *tw = nullptr;            // (cos, sin) per level n = 8 .. N, tier_level_tw; planes by word
   size_t tw_len = 0;                      // entries of a plane
@@ -103,7 +104,6 @@ struct DDeviceTables {
 
 constexpr int kMaxDevices = 64;
 constexpr int kDSubMax = 4096;  // FP64: most points a CTA holds in shared memory (64 KB)
-constexpr int kDSubMin = 64;    // FP64: smallest sub-transform of a longer transform
 // compensated floating-point tiers (float_tier_kernels.cu)
 enum { kTierDD = 0, kTierQD = 1, kTierFF = 2 };
 

@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(256, 2) d_queue_kernel(const QueueItem *__rest
 // compensated tiers: the same pattern
 // ---------------------------------------------------------------------------
 template <class NT, int R>
-__device__ __forceinline__ void tier_queue_upper(const TierTab &S, typename NT::W *out, int lgu, int cols, double scale) {
+__device__ __forceinline__ void tier_queue_upper(const TierTab &S, typename NT::W *out, int lgu, int cols,
+                                                 double scale) {
   for (int t = threadIdx.x; t < cols; t += blockDim.x)
     tier_upper_column<NT, R>(out, S, 1, lgu, 0, t >> lgu, t & ((1 << lgu) - 1), scale, false);
 }
