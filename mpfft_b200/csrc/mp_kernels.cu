@@ -542,11 +542,22 @@ __device__ __forceinline__ void combine_one(int o, bool valid, uint32_t *u0, uin
   }
 }
 
+// CTAs per SM of mp_level_small_kernel: at most eight are ever needed
+// (kSmallLevelButterflies), and up to 8 limbs the 64 registers that leaves are
+// better used than by more of them: left to itself the compiler takes 32 or 40 at 2,
+// 3 and 5 limbs, and the early-scheduled CTAs of the next levels (pdl_release)
+// crowd an SM (us, 32 or 40 registers / this: 3 limbs 64 points x 127 13.1 / 10.2,
+// 256 x 31 17.7 / 14.7; 5 limbs 64 x 127 13.4 / 11.7; 6 limbs 64 x 127 13.5 / 11.7).
+// From 9 limbs it spills (17 limbs 64 x 127 22 / 40): 0, the compiler's choice.
 template <int L>
-__global__ void __launch_bounds__(8 * kSmallBflies) mp_level_small_kernel(uint32_t *__restrict__ y, int N, int B,
-                                                                          int n, const int *__restrict__ node_off,
-                                                                          int nnodes, const uint32_t *__restrict__ twp,
-                                                                          const uint8_t *__restrict__ dneg, int tws) {
+constexpr int small_min_blocks() {
+  return L <= 8 ? 8 : 0;
+}
+
+template <int L>
+__global__ void __launch_bounds__(8 * kSmallBflies, small_min_blocks<L>()) mp_level_small_kernel(
+    uint32_t *__restrict__ y, int N, int B, int n, const int *__restrict__ node_off, int nnodes,
+    const uint32_t *__restrict__ twp, const uint8_t *__restrict__ dneg, int tws) {
   constexpr int Lp = (L + 3) & ~3;
   __shared__ uint32_t Qs[kSmallBflies * 6 * L];  // [butterfly][step][limb]
   pdl_release();
