@@ -469,13 +469,25 @@ static cudaError_t tile_launch(const MpTile &A, cudaStream_t s) {
 static int lg2(long long n) { return 63 - __builtin_clzll((unsigned long long)n); }
 
 // Signals per first-launch tile: the largest power of two up to the room that
-// wastes at most an eighth of the columns.
+// wastes at most an eighth of the columns.  Fewer than 16 signals: the fewest
+// columns, those of one signal counted 3/2 times and of two 11/9 times (rows of
+// one or two words: what they took more, geometric mean over 2 to 33 limbs, 64 to
+// 2^18 points; an eighth at most / this: 3 signals 1 / 0.87, 5 1 / 0.91, 7 1 / 0.78,
+// 9 1 / 0.92, 13 1 / 0.88; from 16 signals on the two differ by less than waves of
+// CTAs do).
 static int tile_lg_signals(int B, int most) {
-  for (int l = most; l > 0; --l) {
-    const long long S = 1LL << l;
-    if ((B + S - 1) / S * S * 8 <= 9LL * B) return l;
+  long long least = 0;
+  int best = 0;
+  for (int l = most; l >= 0; --l) {
+    const long long S = 1LL << l, columns = (B + S - 1) / S * S;
+    if (B >= 16) {
+      if (columns * 8 <= 9LL * B) return l;
+      continue;
+    }
+    const long long cost = columns * (l == 0 ? 27 : l == 1 ? 22 : 18);
+    if (l == most || cost < least) least = cost, best = l;
   }
-  return 0;
+  return best;
 }
 
 template <int L>
@@ -508,9 +520,10 @@ static cudaError_t tile_run(const MpDeviceTables &T, const uint32_t *in, uint32_
 // .. 16384, B = 1 .. 1536 against one launch per level or level pair:
 //   from   a tile's latency is hidden by the others; long single signals, which
 //          take a launch more, last (4 limbs: 4 k points 1.00x, 8 k 1.01 .. 1.15x;
-//          9 limbs: 8 k 0.88 .. 1.06x, 16 k 1.12 .. 1.27x; 12 limbs: 16 k 0.92 ..
-//          1.09x, 20 k 1.16x; 17 limbs 25 k 0.85 .. 1.01x, 33 k 1.05 .. 1.18x; 33
-//          limbs 25 k 0.88 .. 0.98x, 33 k 1.08 .. 1.41x)
+//          9 limbs: 8 k 0.88 .. 1.06x, 12 k 0.93 .. 1.0x for three to seven
+//          signals, 16 k 1.12 .. 1.27x; 12 limbs: 16 k 0.92 .. 1.09x, 20 k 1.16x;
+//          17 limbs 25 k 0.85 .. 1.01x, 33 k 1.05 .. 1.18x; 33 limbs 25 k 0.88 ..
+//          0.98x, 33 k 1.08 .. 1.41x)
 //   to     large batches fill the GPU level by level too, and from 15 limbs up
 //          the register-resident kernels keep more products in flight than a
 //          tile's share of shared memory does (12 limbs 1.5 M points 1.11x, 14 limbs
@@ -520,7 +533,7 @@ static cudaError_t tile_run(const MpDeviceTables &T, const uint32_t *in, uint32_
 bool mp_tile_used(const MpDeviceTables &T, int L, int B) {
   if (!T.twp || L > kMaxLimbs || T.N < 16) return false;
   const long long w = (long long)T.N * B;
-  const long long from = L <= 6 ? 8192 : L <= 9 ? 12288 : L <= 12 ? 20000 : 28672;
+  const long long from = L <= 6 ? 8192 : L <= 9 ? (B < 8 ? 13000 : 12288) : L <= 12 ? 20000 : 28672;
   const long long to = L <= 14   ? (1LL << 62)
                        : L <= 18 ? 1200000
                        : L <= 21 ? 900000

@@ -480,3 +480,26 @@ def test_mp_wide_tiles_bit_identical(M, n, p, B):
         ref = torch.empty_like(one)
         plan.execute_device_timed(1, one.data_ptr(), ref.data_ptr(), s)
         assert torch.equal(d_out[..., b].contiguous(), ref), b
+
+
+@pytest.mark.parametrize("n,p,B", [(1024, 53, 9), (2048, 250, 10), (1024, 380, 13), (2048, 100, 14), (1024, 60, 15),
+                                   (4096, 600, 9), (8192, 1000, 5), (4096, 250, 6), (16384, 760, 3), (32768, 64, 11)])
+def test_mp_tiles_of_few_signals_bit_identical(M, n, p, B):
+    """Batches of fewer than 16 signals, whose tiles may hold rows of more signals
+    than there are: every signal has the bits of its single call."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    plan = M.MpPlan(n, p)
+    L = plan.limbs
+    host = synthetic_planes(n, L, plan.frac_bits, B, seed=n + B).reshape(2, L, n, B)
+    s = torch.cuda.current_stream().cuda_stream
+    d_in = torch.from_numpy(np.ascontiguousarray(host).view(np.int32)).cuda()
+    d_out = torch.full_like(d_in, -1)
+    plan.execute_device(B, d_in.data_ptr(), d_out.data_ptr(), s)
+    for b in range(B):
+        one = d_in[..., b].contiguous()
+        ref = torch.empty_like(one)
+        plan.execute_device_timed(1, one.data_ptr(), ref.data_ptr(), s)
+        assert torch.equal(d_out[..., b].contiguous(), ref), b
