@@ -418,11 +418,15 @@ __device__ void tc_issue(const TcCtx &c, int s) {
 // Tile column n = 8g + r holds output byte column J + g + 16(7 - r), so the
 // limb columns 4(7-r) + j of a tile (j < 4) are in columns 8(4j + e) + r, e < 4.
 // Group q takes the 32 limb columns of tile q of a stage, eight at a time
-// (two adjacent r of every column group).
+// (two adjacent r of every column group); ONE_TILE (nt = 1, a plan forced onto
+// this path at 28 limbs or less, or 30): 16 of the only tile (17 limbs, N=256, batch
+// 256, us, 32 by one group / this: 204 / 179).
+template <bool ONE_TILE>
 __device__ __forceinline__ void tc_product(TcCtx &c, bool valid, uint32_t *dst, size_t ds) {
   const TcGeom &G = c.G;
   const int L = G.L, q = c.q;
-  const uint32_t at = c.tmem + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16) + 128u * q;
+  constexpr int kSeg = ONE_TILE ? 16 : 32;
+  const uint32_t at = c.tmem + ((uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16) + (ONE_TILE ? 0u - 4u * q : 128u * q);
   uint32_t *exL = c.ex, *exC = c.ex + 256, *exT = c.ex + 512;  // low limb, carry-out | ripple, final top limb [2]
   uint32_t carry_in = 0;  // out of the stages so far (< 2^22)
   if (threadIdx.x == 0) {
@@ -430,20 +434,20 @@ __device__ __forceinline__ void tc_product(TcCtx &c, bool valid, uint32_t *dst, 
     tc_issue(c, 0);
   }
   __syncwarp();
-  const int ns = (G.nt + 1) / 2;
+  const int ns = ONE_TILE ? 1 : (G.nt + 1) / 2;
 #pragma unroll 1
   for (int s = 0; s < ns; ++s) {
     if (!c.bad && !mbar_wait(c.bar, c.ph, c.wait_ns)) c.bad = true;
     c.ph ^= 1u;
     tc_fence_after();
-    const int m0 = (G.J0 >> 2) + 64 * s + 32 * q;  // this group's first limb column
-    const bool some = 2 * s + q < G.nt;
-    uint32_t l[32];
+    const int m0 = (G.J0 >> 2) + 2 * kSeg * s + kSeg * q;  // this group's first limb column
+    const bool some = ONE_TILE || 2 * s + q < G.nt;
+    uint32_t l[kSeg];
     uint32_t co = 0;
     if (some) {
       uint64_t cy = 0;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {  // limb columns 8h .. 8h+7: rows r = 7-2h, 6-2h
+      for (int h = 0; h < kSeg / 8; ++h) {  // limb columns 8h .. 8h+7: rows r = 7-2h, 6-2h
         uint32_t v[2][16];
 #pragma unroll
         for (int g = 0; g < 16; ++g) tmem_ld2(at + 8u * g + (6u - 2u * h), v[1][g], v[0][g]);
@@ -462,11 +466,11 @@ __device__ __forceinline__ void tc_product(TcCtx &c, bool valid, uint32_t *dst, 
       co = (uint32_t)cy;
     } else {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) l[i] = 0;
+      for (int i = 0; i < kSeg; ++i) l[i] = 0;
     }
     uint32_t ones = 0xffffffffu;
 #pragma unroll
-    for (int i = 1; i < 32; ++i) ones &= l[i];
+    for (int i = 1; i < kSeg; ++i) ones &= l[i];
     exL[threadIdx.x] = l[0];
     exC[threadIdx.x] = co | (ones == 0xffffffffu ? 0x80000000u : 0u);
     tc_fence_before();
@@ -488,24 +492,24 @@ __device__ __forceinline__ void tc_product(TcCtx &c, bool valid, uint32_t *dst, 
     if (l[0] < cin) {  // rare: cin < 2^22
       l[1] = add_cc(l[1], 1);
 #pragma unroll
-      for (int i = 2; i < 32; ++i) l[i] = addc_cc(l[i], 0);
+      for (int i = 2; i < kSeg; ++i) l[i] = addc_cc(l[i], 0);
     }
     uint32_t *T = exT + (s & 1) * 256;
-    T[threadIdx.x] = l[31];
+    T[threadIdx.x] = l[kSeg - 1];
     __syncthreads();
     if (some && valid) {
       uint32_t prev = q > 0 ? T[c.m] : (s > 0 ? exT[((s - 1) & 1) * 256 + 128 + c.m] : 0u);
       const int i0 = m0 - L;  // result limb of l[0]
       uint32_t *p = dst + (ptrdiff_t)i0 * (ptrdiff_t)ds;
-      if (i0 >= 0 && i0 + 32 <= L) {
+      if (i0 >= 0 && i0 + kSeg <= L) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i, p += ds) {
+        for (int i = 0; i < kSeg; ++i, p += ds) {
           *p = __funnelshift_r(prev, l[i], 31);
           prev = l[i];
         }
       } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i, p += ds) {
+        for (int i = 0; i < kSeg; ++i, p += ds) {
           if (i0 + i >= 0 && i0 + i < L) *p = __funnelshift_r(prev, l[i], 31);
           prev = l[i];
         }
@@ -663,6 +667,7 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 }
 
 // Butterfly k of the node of size n at offset off for signals 128 bg ..
+template <bool ONE_TILE>
 __device__ __forceinline__ void tc_butterfly(TcCtx &c, const TcRun &A, int n, int off, int k, int bg) {
   const int N = A.N, B = A.B, L = A.L, q = n >> 2, grp = c.q;
   uint32_t *y = A.y;
@@ -720,7 +725,7 @@ __device__ __forceinline__ void tc_butterfly(TcCtx &c, const TcRun &A, int n, in
       ds = plane;
     }
     neg |= tc_operand(c, pa, pb, plane, sub, w, tplane) << j;
-    tc_product(c, valid, dst, ds);
+    tc_product<ONE_TILE>(c, valid, dst, ds);
   }
   // merges (T.r from the zi slot, T.i from the zr slot):
   //   Z+: T.r = P + (dn ? R1 : -R1), T.i = P - R2;   Z-: T.r = P + (dn ? -R1 : R1), T.i = R2 - P
@@ -739,6 +744,7 @@ __device__ __forceinline__ void tc_butterfly(TcCtx &c, const TcRun &A, int n, in
   tc_combine(y, P0, P1, u0, u1, z0, z1, c.m, c0, c1, c1, plane, ss, L, t[0], t[1], grp == 0, valid);
 }
 
+template <bool ONE_TILE>
 __global__ void __launch_bounds__(kTcThreads, 2) mp_tc_levels_kernel(const __grid_constant__ TcRun A) {
   extern __shared__ __align__(1024) uint8_t tc_smem[];
   __shared__ int s_item;
@@ -777,7 +783,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) mp_tc_levels_kernel(const __gri
       __threadfence();
     }
     c.bad = __syncthreads_or(c.bad ? 1 : 0) != 0;
-    tc_butterfly(c, A, n, off, k, bg);
+    tc_butterfly<ONE_TILE>(c, A, n, off, k, bg);
     __syncthreads();  // the item's outputs are written (and s_item is read)
     if (threadIdx.x == 0) {
       __threadfence();
@@ -799,7 +805,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   TcCtx c;
   tc_setup(c, tc_smem, L);
   const uint32_t neg = tc_operand(c, x + bs, nullptr, (size_t)B, false, w, 1);
-  tc_product(c, valid, out + bs, (size_t)B);
+  tc_product<false>(c, valid, out + bs, (size_t)B);
   __syncthreads();
   if (valid && neg && threadIdx.x < kTcRows) {
     uint32_t cy = 1;
@@ -911,7 +917,8 @@ cudaError_t mp_tc_run_levels(int L, const MpDeviceTables &T, uint32_t *out, int 
   if (T.nlevels == 0) return cudaSuccess;
   const TcGeom G = tc_geom(L);
   int *err = nullptr;
-  cudaError_t e = tc_prepare((const void *)mp_tc_levels_kernel, G.bytes, &err);
+  const auto kernel = G.nt == 1 ? mp_tc_levels_kernel<true> : mp_tc_levels_kernel<false>;
+  cudaError_t e = tc_prepare((const void *)kernel, G.bytes, &err);
   if (e != cudaSuccess) return e;
   const int ctas = tc_ctas(T, B);
   TcRun A{};
@@ -946,7 +953,7 @@ cudaError_t mp_tc_run_levels(int L, const MpDeviceTables &T, uint32_t *out, int 
     timer.begin();
     e = step == 1 ? cudaMemsetAsync(A.head, 0, sizeof(int), s) : cudaMemsetAsync(A.flags, 0, fw * 4, s);
     if (e != cudaSuccess) break;
-    mp_tc_levels_kernel<<<(unsigned)std::min<long long>(ctas, A.first[A.lv1]), kTcThreads, G.bytes, s>>>(A);
+    kernel<<<(unsigned)std::min<long long>(ctas, A.first[A.lv1]), kTcThreads, G.bytes, s>>>(A);
     timer.end();
     e = cudaGetLastError();
   }

@@ -158,3 +158,41 @@ def test_tc_segment_carries(M):
             got = _from_planes(y.cpu().numpy().view(np.uint32))
             for v, g in zip(xs, got):
                 assert g == _tc_expected(v, w, L), (L, hex(v)[:20], hex(w)[:20])
+
+
+@pytest.mark.parametrize("L", [8, 9, 13, 14, 17, 21, 25, 28, 29, 30, 31, 34])
+@pytest.mark.parametrize("n,B", [(8, 3), (64, 1), (64, 130)])
+def test_tc_forced_below_its_default_range(M, L, n, B):
+    """Plans forced onto the tensor cores (one tile of byte columns up to 28 limbs
+    and at 30, two at 29 and from 31) against the integer pipe: both round each
+    product to within a unit of the last place.  A difference e of a level's inputs
+    becomes at most (2e + 1) + (sqrt 2 e + 1) in a twiddled value, twice that in
+    their sum, plus e: 8e + 4.  Signals cut from the batch have the batch's bits."""
+    import torch
+
+    from mpfft_b200.mparray import synthetic_planes
+
+    lg = n.bit_length() - 1
+    plan = M.MpPlan(n, 32 * L - 7 - 2 * lg, tensor="force")
+    ref = M.MpPlan(n, 32 * L - 7 - 2 * lg, tensor=False)
+    assert plan.limbs == ref.limbs == L and plan.form() != ref.form()
+    host = synthetic_planes(n, L, plan.frac_bits, B, seed=n + L).reshape(2, L, n, B)
+    s = torch.cuda.current_stream().cuda_stream
+    d_in = torch.from_numpy(np.ascontiguousarray(host).view(np.int32)).cuda()
+    a, b = torch.full_like(d_in, -1), torch.full_like(d_in, -1)
+    plan.execute_device(B, d_in.data_ptr(), a.data_ptr(), s)
+    ref.execute_device(B, d_in.data_ptr(), b.data_ptr(), s)
+    for i in {0, B - 1}:
+        one = d_in[..., i].contiguous()
+        out = torch.empty_like(one)
+        plan.execute_device(1, one.data_ptr(), out.data_ptr(), s)
+        assert torch.equal(out, a[..., i].contiguous()), i
+    M.tc_error()
+    bound = 0
+    for _ in range(lg - 2):  # levels n = 8 ..
+        bound = 8 * bound + 4
+    ints = lambda t: np.ascontiguousarray(t.cpu().numpy().view(np.uint32).transpose(0, 2, 3, 1)).reshape(-1, L)
+    top = 1 << (32 * L)
+    for x, y in zip(ints(a), ints(b)):
+        d = (int.from_bytes(x.tobytes(), "little") - int.from_bytes(y.tobytes(), "little")) % top
+        assert min(d, top - d) <= bound, (hex(d), bound)
